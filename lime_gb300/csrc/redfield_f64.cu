@@ -15,6 +15,9 @@
 // the exact path (DFMA-bound on GB300).
 
 #include "gemm_f64.cuh"
+#include "redfield_vec_f64.cuh"
+
+#include <math.h>
 
 namespace lime {
 namespace rf {
@@ -79,19 +82,39 @@ __global__ void __launch_bounds__(kThreads) assemble_kernel(BuildArgs a) {
   gemm_tile(D, D, 2 * K, blockIdx.y * kTile, blockIdx.x * kTile, la, lb, epi);
 }
 
-// obs[r][o] = sum_ij E_o[j][i] rho_r[i][j]  (D-dot per observable and RHS)
-__global__ void observe_kernel(int n, int R, int n_obs, const double2* Eops, const double2* P, double2* out) {
-  const int64_t D = (int64_t)n * n;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)R * n_obs;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(t / n_obs), o = (int)(t % n_obs);
+// out[slot][r][o] = sum_ij E_o[j][i] rho_r[i][j] over kept states hist[slot][D][R],
+// one warp each: D / 32 terms a lane, where one thread summing all D left the
+// chip idle for 144 us a step at D = 400
+__global__ void observe_kernel(int n, int R, int n_obs, int slots, const double2* Eops, const double2* hist,
+                               double2* out) {
+  const int64_t D = (int64_t)n * n, total = (int64_t)slots * R * n_obs;
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t t = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); t < total; t += nw) {
+    const int o = (int)(t % n_obs);
+    const int64_t sr = t / n_obs;
+    const int r = (int)(sr % R);
+    const double2* P = hist + (sr / R) * D * R + r;
     double2 s = cz();
-    for (int64_t e = 0; e < D; ++e) {
-      const int i = (int)(e / n), j = (int)(e % n);
-      cfma(s, Eops[o * D + (int64_t)j * n + i], P[e * R + r]);
+    for (int64_t e = lane; e < D; e += 32) {
+      const int64_t j = e / n, i = e - j * n;
+      cfma(s, Eops[o * D + e], P[(i * n + j) * R]);
     }
-    out[(int64_t)r * n_obs + o] = s;
+    for (int w = 16; w > 0; w >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, w);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, w);
+    }
+    if (lane == 0) out[t] = s;
   }
+}
+
+static int observe(int n, int R, int n_obs, int slots, const double2* E, const double2* hist, double2* out,
+                   cudaStream_t st) {
+  const int64_t warps = (int64_t)slots * R * n_obs, blocks = (warps + 3) / 4;
+  observe_kernel<<<(unsigned)(blocks < 65535 ? blocks : 65535), 128, 0, st>>>(n, R, n_obs, slots, E, hist, out);
+  LIME_CUDA_TRY(cudaGetLastError());
+  count_launch();
+  return LIME_OK;
 }
 
 }  // namespace rf
@@ -149,7 +172,47 @@ extern "C" int lime_redfield_assemble_f64(const LimeRedfieldAssembleDesc* d, voi
 
 extern "C" size_t lime_redfield_rk4_f64_workspace(int32_t n, int32_t n_rhs) {
   if (n <= 0 || n_rhs <= 0) return 0;
-  return (size_t)3 * n * n * n_rhs * sizeof(double2);
+  const size_t tiled = (size_t)3 * n * n * n_rhs * sizeof(double2);
+  if ((int64_t)n * n > 46340 || !rfv::supported(n * n, n_rhs)) return tiled;
+  return tiled + rfv::workspace(n * n, n_rhs);
+}
+
+// The time loop in single launches: a chunk is as many steps as the kept
+// states have slots for, and at most about a tenth of a second of FP64 work.
+static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, cudaStream_t st) {
+  const int n = d->n, D = n * n, R = d->n_rhs;
+  const size_t DR = (size_t)D * R;
+  const int obs_every = d->obs_every > 0 ? d->obs_every : 1;
+  rfv::Run r{};
+  r.D = D; r.R = R; r.n_steps = d->n_steps; r.dt = d->dt;
+  r.L = reinterpret_cast<const double2*>(d->R);
+  r.P = reinterpret_cast<double2*>(d->rho);
+  r.ws = reinterpret_cast<double2*>(d->workspace) + 3 * DR;
+  r.states = reinterpret_cast<double2*>(d->states); r.states_every = d->states_every;
+  r.obs_every = d->n_obs > 0 ? obs_every : 0;
+  // the caller's states serve the observables when they are the same steps
+  const bool own = d->n_obs > 0 && !(d->states && d->states_every == obs_every);
+  double2* out = reinterpret_cast<double2*>(d->obs_out);
+  const double2* E = reinterpret_cast<const double2*>(d->obs_ops);
+  int rc = rfv::begin(plan, r, st);
+  if (rc != LIME_OK) return rc;
+  const double per_step = 16.0 * D * (double)D * R;
+  int64_t chunk = (int64_t)fmax(1.0, fmin((double)d->n_steps, 5e10 / per_step));
+  if (own && chunk > (int64_t)rfv::kHistory * obs_every) chunk = (int64_t)rfv::kHistory * obs_every;
+  for (int64_t s0 = 0; s0 < d->n_steps; s0 += chunk) {
+    const int steps = (int)(d->n_steps - s0 < chunk ? d->n_steps - s0 : chunk);
+    double2* hist = own ? rfv::history(r) : nullptr;
+    rc = rfv::launch(plan, r, (int)s0, steps, hist, st);
+    if (rc != LIME_OK) return rc;
+    const int64_t k0 = s0 / obs_every, slots = (s0 + steps) / obs_every - k0;
+    if (own && slots > 0) {
+      rc = rf::observe(n, R, d->n_obs, (int)slots, E, hist, out + k0 * R * d->n_obs, st);
+      if (rc != LIME_OK) return rc;
+    }
+  }
+  if (d->n_obs > 0 && !own && d->n_steps / obs_every > 0)
+    return rf::observe(n, R, d->n_obs, d->n_steps / obs_every, E, r.states, out, st);
+  return LIME_OK;
 }
 
 extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream) {
@@ -158,16 +221,26 @@ extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream)
   if (d->n_obs > 0 && (!d->obs_ops || !d->obs_out)) return LIME_ERR_ARG;
   if (d->states && d->states_every <= 0) return LIME_ERR_ARG;
   if ((int64_t)d->n * d->n > 46340) return LIME_ERR_UNSUPPORTED;
-  if (d->workspace_bytes < lime_redfield_rk4_f64_workspace(d->n, d->n_rhs)) return LIME_ERR_WORKSPACE;
-  cudaStream_t st = (cudaStream_t)stream;
   const int D = d->n * d->n, R = d->n_rhs;
   const size_t DR = (size_t)D * R;
+  if (d->workspace_bytes < 3 * DR * sizeof(double2)) return LIME_ERR_WORKSPACE;
+  cudaStream_t st = (cudaStream_t)stream;
+  // Few right-hand sides: one launch for the time loop, where the workspace
+  // has room for its exchange (a caller that sized it for the tiled path
+  // alone stays there).  From kMaxRhs right-hand sides on a tile's columns
+  // are used and the tiled GEMM is as near to the FP64 bound.
+  if (d->n_steps > 0 && d->workspace_bytes >= lime_redfield_rk4_f64_workspace(d->n, R)) {
+    int dev = 0, sms = 0;
+    LIME_CUDA_TRY(cudaGetDevice(&dev));
+    LIME_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    rfv::Plan plan;
+    if (rfv::plan(D, R, sms, &plan)) return rk4_vec(d, plan, st);
+  }
   double2* P = reinterpret_cast<double2*>(d->rho);
   double2* acc = reinterpret_cast<double2*>(d->workspace);
   double2* S0 = acc + DR;
   double2* S1 = S0 + DR;
   const int obs_every = d->obs_every > 0 ? d->obs_every : 1;
-  const int n_slots = d->n_steps / obs_every;
   dim3 grid((R + rf::kTile - 1) / rf::kTile, (D + rf::kTile - 1) / rf::kTile);
   int64_t launches = 0;
   for (int step = 0; step < d->n_steps; ++step) {
@@ -182,20 +255,16 @@ extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream)
     }
     if (d->n_obs > 0 && ((step + 1) % obs_every) == 0) {
       const int slot = (step + 1) / obs_every - 1;
-      double2* tmp = reinterpret_cast<double2*>(d->obs_out);
       // obs_out layout [slot][R][n_obs]
-      const int tb = (R * d->n_obs + 127) / 128;
-      rf::observe_kernel<<<tb, 128, 0, st>>>(d->n, R, d->n_obs, reinterpret_cast<const double2*>(d->obs_ops), P,
-                                             tmp + (size_t)slot * R * d->n_obs);
-      LIME_CUDA_TRY(cudaGetLastError());
-      ++launches;
+      const int rc = rf::observe(d->n, R, d->n_obs, 1, reinterpret_cast<const double2*>(d->obs_ops), P,
+                                 reinterpret_cast<double2*>(d->obs_out) + (size_t)slot * R * d->n_obs, st);
+      if (rc != LIME_OK) return rc;
     }
     if (d->states && ((step + 1) % d->states_every) == 0) {
       const int slot = (step + 1) / d->states_every - 1;
       LIME_CUDA_TRY(cudaMemcpyAsync(reinterpret_cast<double2*>(d->states) + (size_t)slot * DR, P,
                                     DR * sizeof(double2), cudaMemcpyDeviceToDevice, st));
     }
-    (void)n_slots;
   }
   count_launch(launches);
   return LIME_OK;
