@@ -1,14 +1,23 @@
 // Batched complex128 discrete Fourier transforms for the spectra of
 // propagated correlation functions (lime/fft.py:9-56: g(w) = fftshift(fft(f))
 // dx exp(-i w x0)).  Power-of-two lengths up to 8192 run as one CTA per
-// transform, radix-2 decimation in time entirely in shared memory (inputs
-// loaded in bit-reversed order, log2 n butterfly stages, twiddles from
-// sincospi); other lengths up to 4096 go through Bluestein's chirp-z
-// identity
+// transform, decimation in time with three radix-2 stages a pass in
+// registers and one exchange through shared memory between passes; the first
+// pass reads global memory, the last one writes it.  Other lengths up to 4096
+// go through Bluestein's chirp-z identity
 //     X_k = c_k sum_j (x_j c_j) conj(c_{k-j}),   c_j = exp(-i pi j^2 / n)
-// as a circular convolution of length m = 2^ceil(log2(2n - 1)) (three
-// power-of-two transforms).  The output can be written fftshift-ed and
-// multiplied by a per-position factor (dx exp(-i w_k x0) for lime's fft).
+// as a circular convolution of length m = 2^ceil(log2(2n - 1)): the chirp, the
+// forward transforms (the filter's among them) and the inverse transforms are
+// a launch each.  The output can be written fftshift-ed and multiplied by a
+// per-position factor (dx exp(-i w_k x0) for lime's fft).
+//
+// Bound: the FP64 pipe (1.68 lanes per clock and SM; everything else is
+// nearly free beside it), so the butterflies are counted in FP64
+// instructions: u + w v and 2 u - (u + w v) are 6 fma, the first pass's
+// factors 1 and -i are 4 additions, and the factors come from a table that
+// the compiler fills (a sincospi in each butterfly took 40 of 48).  256
+// transforms of 4096: 722 -> 93 us, 33.5 + 4 FP64 instructions a point being
+// 78 us; 100 of length 999: 504 -> 51 us in the transforms, 3 launches for 6.
 
 #include "common.cuh"
 
@@ -17,92 +26,229 @@ namespace fft {
 
 constexpr int kThreads = 512;
 constexpr int kMaxPow2 = 8192;
+constexpr int kRoots = kMaxPow2 / 2;
+
+// exp(-2 pi i j / 8192), j = 0 .. 4095, from the Taylor series of the first
+// octant in 62-bit fixed point (error under 2^-59), rounded once
+struct Roots {
+  double v[2 * kRoots];
+};
+constexpr long long fixmul(long long a, long long b) { return (long long)(((__int128)a * b) >> 62); }
+constexpr Roots make_roots() {
+  Roots r{};
+  const unsigned long long pi = 0xC90FDAA22168C235ull;   // pi 2^62
+  for (int j = 0; j <= kRoots / 4; ++j) {
+    const long long x = (long long)(((unsigned __int128)pi * (unsigned)j) >> 12);   // 2 pi j / 8192
+    const long long x2 = fixmul(x, x);
+    long long c = 1ll << 62, s = x, tc = c, ts = x;
+    for (int k = 1; k <= 11; ++k) {
+      tc = -fixmul(tc, x2) / ((2 * k - 1) * (2 * k));
+      ts = -fixmul(ts, x2) / ((2 * k) * (2 * k + 1));
+      c += tc;
+      s += ts;
+    }
+    const double one = 4611686018427387904.0;   // 2^62
+    const double cd = (double)c / one, sd = (double)s / one;
+    // octants: (c, -s) at j; (s, -c) at 2048 - j; (-s, -c) at 2048 + j; (-c, -s) at 4096 - j
+    const int h = kRoots / 2;
+    r.v[2 * j] = cd;
+    r.v[2 * j + 1] = -sd;
+    r.v[2 * (h - j)] = sd;
+    r.v[2 * (h - j) + 1] = -cd;
+    r.v[2 * (h + j)] = -sd;
+    r.v[2 * (h + j) + 1] = -cd;
+    if (j > 0) {
+      r.v[2 * (kRoots - j)] = -cd;
+      r.v[2 * (kRoots - j) + 1] = -sd;
+    }
+  }
+  r.v[1] = 0.0;
+  r.v[kRoots] = 0.0;
+  return r;
+}
+__device__ const Roots g_roots = make_roots();
+
+__device__ __forceinline__ double2 root(int j) { return reinterpret_cast<const double2*>(g_roots.v)[j]; }
+__device__ __forceinline__ unsigned bitrev(unsigned v, int bits) { return bits == 0 ? 0u : __brev(v) >> (32 - bits); }
+// place of element i in shared memory: the low three bits take in the higher
+// ones, so that the bit-reversed stores of the first pass (one low part for
+// all lanes) spread over the banks
+__device__ __forceinline__ int sw(int i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9)) & 7); }
+
+// (u, v) <- (u + w v, u - w v)
+__device__ __forceinline__ void bfly(double2& u, double2& v, double2 w) {
+  const double2 r = make_double2(fma(-w.y, v.y, fma(w.x, v.x, u.x)), fma(w.y, v.x, fma(w.x, v.y, u.y)));
+  v = make_double2(fma(2.0, u.x, -r.x), fma(2.0, u.y, -r.y));
+  u = r;
+}
+// with -i w
+__device__ __forceinline__ void bfly_mi(double2& u, double2& v, double2 w) { bfly(u, v, make_double2(w.y, -w.x)); }
+__device__ __forceinline__ void bfly_1(double2& u, double2& v) {
+  const double2 r = cadd(u, v);
+  v = csub(u, v);
+  u = r;
+}
+__device__ __forceinline__ void bfly_mi1(double2& u, double2& v) {
+  const double2 r = make_double2(u.x + v.y, u.y - v.x);
+  v = make_double2(u.x - v.y, u.y + v.x);
+  u = r;
+}
+
+// the first K stages of 2^K elements (factors exp(-i pi m / 2^stage))
+template <int K>
+__device__ __forceinline__ void first_stages(double2 (&v)[8]) {
+#pragma unroll
+  for (int m = 0; m < (1 << K); m += 2) bfly_1(v[m], v[m + 1]);
+  if (K > 1)
+#pragma unroll
+    for (int m = 0; m < (1 << K); m += 4) {
+      bfly_1(v[m], v[m + 2]);
+      bfly_mi1(v[m + 1], v[m + 3]);
+    }
+  if (K > 2) {
+    const double2 w = root(kRoots / 4);
+    bfly_1(v[0], v[4]);
+    bfly(v[1], v[5], w);
+    bfly_mi1(v[2], v[6]);
+    bfly_mi(v[3], v[7], w);
+  }
+}
+
+template <int K, class Load, class Store>
+__device__ __forceinline__ void first_pass(double2* s, int L, const Load& load, const Store& store) {
+  const int groups = 1 << (L - K);
+  for (int r = threadIdx.x; r < groups; r += blockDim.x) {
+    double2 v[8];
+#pragma unroll
+    for (int m = 0; m < (1 << K); ++m) v[m] = load((int)(__brev((unsigned)m) >> (32 - K)) * groups + r);
+    first_stages<K>(v);
+    const int q = (int)bitrev((unsigned)r, L - K);
+#pragma unroll
+    for (int m = 0; m < (1 << K); ++m) {
+      if (L == K) store(m, v[m]);
+      else s[sw((q << K) + m)] = v[m];
+    }
+  }
+}
+
+// y_k = sum_j load(j) exp(-2 pi i j k / 2^L), store(k, y_k), by one CTA; s: 2^L elements
+template <class Load, class Store>
+__device__ void transform(double2* s, int L, const Load& load, const Store& store) {
+  const int n = 1 << L;
+  if (L == 0) {
+    if (threadIdx.x == 0) store(0, load(0));
+    return;
+  }
+  const int K = L % 3 == 0 ? 3 : L % 3;
+  if (K == 3) first_pass<3>(s, L, load, store);
+  else if (K == 2) first_pass<2>(s, L, load, store);
+  else first_pass<1>(s, L, load, store);
+  for (int h = 1 << K, lh = K; h < n; h <<= 3, lh += 3) {
+    __syncthreads();
+    const bool last = h << 3 == n;
+    for (int q = threadIdx.x; q < n >> 3; q += blockDim.x) {
+      const int pos = q & (h - 1), base = ((q - pos) << 3) + pos;
+      // factors of the stages of half length h, 2 h, 4 h at pos
+      const int j3 = pos << (10 - lh);
+      const double2 w1 = root(j3 << 2), w2 = root(j3 << 1), w3 = root(j3), w3a = root(j3 + kRoots / 4);
+      double2 v[8];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) v[m] = s[sw(base + (m << lh))];
+#pragma unroll
+      for (int m = 0; m < 8; m += 2) bfly(v[m], v[m + 1], w1);
+#pragma unroll
+      for (int m = 0; m < 8; m += 4) {
+        bfly(v[m], v[m + 2], w2);
+        bfly_mi(v[m + 1], v[m + 3], w2);
+      }
+      bfly(v[0], v[4], w3);
+      bfly(v[1], v[5], w3a);
+      bfly_mi(v[2], v[6], w3);
+      bfly_mi(v[3], v[7], w3a);
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        if (last) store(base + (m << lh), v[m]);
+        else s[sw(base + (m << lh))] = v[m];
+      }
+    }
+  }
+}
 
 struct Pass {
-  int n, log2n, inverse;
+  int n, log2n;              // transform length (Bluestein: the convolution's m)
+  int len, inverse;          // data length, sign of the transform
   const double2* x; int64_t x_s, x_bs;
   double2* y; int64_t y_s, y_bs;
-  int shift;                 // write output k at (k + n/2) % n
+  int shift;                 // write output k at (k + len/2) % len
   const double2* post;       // per output position factor (after the shift), or null
-  const double2* mul;        // per frequency factor applied before the store (Bluestein's B_k), or null
-  double scale;
+  double2* conv;             // Bluestein: [batch][m]
+  double2* chirp;            // Bluestein: c_j, j < len, then the filter's spectrum k = 0 .. m/2
 };
 
-__device__ __forceinline__ unsigned bitrev(unsigned v, int bits) { return bits == 0 ? 0u : __brev(v) >> (32 - bits); }
+// an inverse transform is the conjugate of the transform of the conjugate
+__device__ __forceinline__ double2 conj_if(double2 v, int on) { return on ? cconj(v) : v; }
+
+__device__ __forceinline__ void put(const Pass& p, int64_t b, int k, double2 v) {
+  int ks = k;
+  if (p.shift) {
+    ks = k + p.len / 2;
+    if (ks >= p.len) ks -= p.len;
+  }
+  if (p.post) v = cmul(v, p.post[ks]);
+  p.y[b * p.y_bs + (int64_t)ks * p.y_s] = v;
+}
 
 __global__ void __launch_bounds__(kThreads) pow2_kernel(Pass p) {
   extern __shared__ double2 s[];
-  const int n = p.n;
   const int64_t b = blockIdx.x;
   const double2* x = p.x + b * p.x_bs;
-  for (int j = threadIdx.x; j < n; j += kThreads) s[bitrev((unsigned)j, p.log2n)] = x[(int64_t)j * p.x_s];
-  __syncthreads();
-  const double sgn = p.inverse ? 1.0 : -1.0;
-  for (int half = 1; half < n; half <<= 1) {
-    for (int q = threadIdx.x; q < n / 2; q += kThreads) {
-      const int pos = q & (half - 1);
-      const int i0 = ((q - pos) << 1) + pos, i1 = i0 + half;
-      double sn, cs;
-      sincospi(sgn * (double)pos / (double)half, &sn, &cs);   // exp(-+ i pi pos / half)
-      const double2 u = s[i0], v = s[i1];
-      const double2 w = make_double2(v.x * cs - v.y * sn, v.x * sn + v.y * cs);
-      s[i0] = make_double2(u.x + w.x, u.y + w.y);
-      s[i1] = make_double2(u.x - w.x, u.y - w.y);
-    }
-    __syncthreads();
-  }
-  double2* y = p.y + b * p.y_bs;
-  for (int k = threadIdx.x; k < n; k += kThreads) {
-    double2 v = s[k];
-    if (p.mul) v = cmul(v, p.mul[k]);
-    v = cscale(v, p.scale);
-    const int ks = p.shift ? (k + n / 2) % n : k;
-    if (p.post) v = cmul(v, p.post[ks]);
-    y[(int64_t)ks * p.y_s] = v;
-  }
+  transform(s, p.log2n, [&](int j) { return conj_if(x[(int64_t)j * p.x_s], p.inverse); },
+            [&](int k, double2 v) { put(p, b, k, conj_if(v, p.inverse)); });
 }
 
-// exp(sgn i pi j^2 / n) with the argument reduced exactly (j^2 mod 2n)
-__device__ __forceinline__ double2 chirp(int64_t j, int n, double sgn) {
-  const int64_t r = (j * j) % (2 * (int64_t)n);
+// c_j = exp(-+ i pi j^2 / len), the argument reduced exactly (j^2 mod 2 len)
+__global__ void chirp_kernel(Pass p) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= p.len) return;
+  const int64_t r = ((int64_t)j * j) % (2 * (int64_t)p.len);
   double sn, cs;
-  sincospi(sgn * (double)r / (double)n, &sn, &cs);
-  return make_double2(cs, sn);
+  sincospi((double)r / (double)p.len, &sn, &cs);
+  p.chirp[j] = make_double2(cs, p.inverse ? sn : -sn);
 }
 
-// a[b][j] = x[b][j] c_j (j < n), 0 up to m
-__global__ void chirp_in_kernel(const double2* x, int64_t x_s, int64_t x_bs, int n, int m, int batch, double sgn,
-                                double2* a) {
-  const int64_t total = (int64_t)batch * m;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = e / m;
-    const int j = (int)(e - b * m);
-    a[e] = j < n ? cmul(x[b * x_bs + (int64_t)j * x_s], chirp(j, n, sgn)) : cz();
+// block b < batch: the spectrum of x_j c_j; the last block: half the
+// spectrum of the filter conj(c_j), wrapped circularly (even, so its spectrum
+// is too, and with the chirp it fits one row of the workspace)
+__global__ void __launch_bounds__(kThreads) chirp_forward_kernel(Pass p) {
+  extern __shared__ double2 s[];
+  const int64_t b = blockIdx.x;
+  const int len = p.len, m = p.n;
+  if (b + 1 == gridDim.x) {
+    double2* spec = p.chirp + len;
+    transform(s, p.log2n,
+              [&](int j) {
+                const int k = j < len ? j : j > m - len ? m - j : -1;
+                return k < 0 ? cz() : cconj(p.chirp[k]);
+              },
+              [&](int k, double2 v) { if (2 * k <= m) spec[k] = v; });
+    return;
   }
+  const double2* x = p.x + b * p.x_bs;
+  double2* c = p.conv + b * m;
+  transform(s, p.log2n, [&](int j) { return j < len ? cmul(x[(int64_t)j * p.x_s], p.chirp[j]) : cz(); },
+            [&](int k, double2 v) { c[k] = v; });
 }
 
-// the chirp filter conj(c_m), wrapped circularly into length m
-__global__ void chirp_filter_kernel(int n, int m, double sgn, double2* f) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-    double2 v = cz();
-    if (k < n) v = chirp(k, n, -sgn);
-    else if (k > m - n) v = chirp(m - k, n, -sgn);
-    f[k] = v;
-  }
-}
-
-// X_k = c_k conv_k / m, written (shifted, times post) to y
-__global__ void chirp_out_kernel(const double2* conv, int n, int m, int batch, double sgn, int shift,
-                                 const double2* post, double2* y, int64_t y_s, int64_t y_bs) {
-  const int64_t total = (int64_t)batch * n;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = e / n;
-    const int k = (int)(e - b * n);
-    double2 v = cscale(cmul(conv[b * m + k], chirp(k, n, sgn)), 1.0 / (double)m);
-    const int ks = shift ? (k + n / 2) % n : k;
-    if (post) v = cmul(v, post[ks]);
-    y[b * y_bs + (int64_t)ks * y_s] = v;
-  }
+// X_k = c_k conv_k / m from the product of the spectra
+__global__ void __launch_bounds__(kThreads) chirp_inverse_kernel(Pass p) {
+  extern __shared__ double2 s[];
+  const int64_t b = blockIdx.x;
+  const int len = p.len, m = p.n;
+  const double2* c = p.conv + b * m;
+  const double2* spec = p.chirp + len;
+  const double scale = 1.0 / (double)m;   // a power of two
+  transform(s, p.log2n, [&](int k) { return cconj(cmul(c[k], spec[2 * k <= m ? k : m - k])); },
+            [&](int k, double2 v) { if (k < len) put(p, b, k, cmul(cscale(cconj(v), scale), p.chirp[k])); });
 }
 
 int log2_exact(int n) {
@@ -134,57 +280,37 @@ extern "C" int lime_fft_f64(const LimeFftDesc* d, void* stream) {
   if ((d->inverse & ~1) || (d->shift & ~1)) return LIME_ERR_ARG;
   const int n = d->n;
   cudaStream_t st = (cudaStream_t)stream;
-  const double sgn = d->inverse ? 1.0 : -1.0;
-  const size_t smem_max = (size_t)fft::kMaxPow2 * sizeof(double2);
-  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::pow2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
   const int l2 = fft::log2_exact(n);
+  const int m = l2 >= 0 ? n : fft::bluestein_len(n);
+  if (m > fft::kMaxPow2) return LIME_ERR_UNSUPPORTED;
+  if (l2 < 0 && (!d->workspace || d->workspace_bytes < lime_fft_f64_workspace(n, d->batch)))
+    return LIME_ERR_WORKSPACE;
+  fft::Pass p{};
+  p.n = m; p.log2n = fft::log2_exact(m); p.len = n; p.inverse = d->inverse;
+  p.x = reinterpret_cast<const double2*>(d->x); p.x_s = d->x_s; p.x_bs = d->x_bs;
+  p.y = reinterpret_cast<double2*>(d->y); p.y_s = d->y_s; p.y_bs = d->y_bs;
+  p.shift = d->shift;
+  p.post = reinterpret_cast<const double2*>(d->post);
+  const size_t smem = (size_t)m * sizeof(double2);
+  // a thread takes 8 elements of a pass
+  const int nt = m / 8 < 32 ? 32 : m / 8 < fft::kThreads ? m / 8 : fft::kThreads;
   if (l2 >= 0) {
-    if (n > fft::kMaxPow2) return LIME_ERR_UNSUPPORTED;
-    fft::Pass p{};
-    p.n = n; p.log2n = l2; p.inverse = d->inverse;
-    p.x = reinterpret_cast<const double2*>(d->x); p.x_s = d->x_s; p.x_bs = d->x_bs;
-    p.y = reinterpret_cast<double2*>(d->y); p.y_s = d->y_s; p.y_bs = d->y_bs;
-    p.shift = d->shift;
-    p.post = reinterpret_cast<const double2*>(d->post);
-    p.scale = 1.0;
-    fft::pow2_kernel<<<d->batch, fft::kThreads, (size_t)n * sizeof(double2), st>>>(p);
+    LIME_CUDA_TRY(cudaFuncSetAttribute(fft::pow2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    fft::pow2_kernel<<<d->batch, nt, smem, st>>>(p);
     LIME_CUDA_TRY(cudaGetLastError());
     count_launch();
     return LIME_OK;
   }
-  const int m = fft::bluestein_len(n);
-  if (m > fft::kMaxPow2) return LIME_ERR_UNSUPPORTED;
-  if (!d->workspace || d->workspace_bytes < lime_fft_f64_workspace(n, d->batch)) return LIME_ERR_WORKSPACE;
-  double2* a = reinterpret_cast<double2*>(d->workspace);     // [batch][m]
-  double2* f = a + (size_t)d->batch * m;                      // [m]
-  const int lm = fft::log2_exact(m);
-  const int64_t tot = (int64_t)d->batch * m;
-  const int gb = (int)((tot + 255) / 256 < 65535 ? (tot + 255) / 256 : 65535);
-  fft::chirp_in_kernel<<<gb, 256, 0, st>>>(reinterpret_cast<const double2*>(d->x), d->x_s, d->x_bs, n, m, d->batch,
-                                           sgn, a);
+  p.conv = reinterpret_cast<double2*>(d->workspace);      // [batch][m]
+  p.chirp = p.conv + (size_t)d->batch * m;                 // [m]: n + m/2 + 1 <= m, n is not a power of two
+  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::chirp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::chirp_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fft::chirp_kernel<<<(n + 63) / 64, 64, 0, st>>>(p);
   LIME_CUDA_TRY(cudaGetLastError());
-  fft::chirp_filter_kernel<<<(m + 255) / 256, 256, 0, st>>>(n, m, sgn, f);
+  fft::chirp_forward_kernel<<<d->batch + 1, nt, smem, st>>>(p);
   LIME_CUDA_TRY(cudaGetLastError());
-  fft::Pass p{};
-  p.n = m; p.log2n = lm; p.scale = 1.0;
-  // F = FFT(filter), in place
-  p.inverse = 0; p.x = f; p.x_s = 1; p.x_bs = m; p.y = f; p.y_s = 1; p.y_bs = m;
-  fft::pow2_kernel<<<1, fft::kThreads, (size_t)m * sizeof(double2), st>>>(p);
+  fft::chirp_inverse_kernel<<<d->batch, nt, smem, st>>>(p);
   LIME_CUDA_TRY(cudaGetLastError());
-  // A = FFT(a) * F, in place
-  p.x = a; p.y = a; p.mul = f;
-  fft::pow2_kernel<<<d->batch, fft::kThreads, (size_t)m * sizeof(double2), st>>>(p);
-  LIME_CUDA_TRY(cudaGetLastError());
-  // conv = IFFT(A) (unscaled), in place
-  p.inverse = 1; p.mul = nullptr;
-  fft::pow2_kernel<<<d->batch, fft::kThreads, (size_t)m * sizeof(double2), st>>>(p);
-  LIME_CUDA_TRY(cudaGetLastError());
-  const int64_t tn = (int64_t)d->batch * n;
-  const int go = (int)((tn + 255) / 256 < 65535 ? (tn + 255) / 256 : 65535);
-  fft::chirp_out_kernel<<<go, 256, 0, st>>>(a, n, m, d->batch, sgn, d->shift,
-                                            reinterpret_cast<const double2*>(d->post),
-                                            reinterpret_cast<double2*>(d->y), d->y_s, d->y_bs);
-  LIME_CUDA_TRY(cudaGetLastError());
-  count_launch(6);
+  count_launch(3);
   return LIME_OK;
 }
