@@ -20,8 +20,8 @@
 // Bound: 4 D^2 R DFMA a stage at 1.68 lanes per clock and SM, and the latency
 // of the exchange.  Measured against one 64 x 64 tiled GEMM launch a stage
 // (one CTA per 64 rows, 63 of 64 columns padding), one right-hand side: D =
-// 400 (kGrid), 100 steps with everything a call does, 669 -> 3.0 ms; D = 36
-// (kCluster) 198 -> 2.0 us a stage.
+// 400 (kGrid) 1632 -> 3.7 us a stage, of which the DFMA are 1.3; D = 36
+// (kCluster) 198 -> 2.0 us.
 
 #include "redfield_vec_f64.cuh"
 

@@ -8,7 +8,9 @@
 // scale s (the exp(w_j t_z) of the spectral propagator), and arbitrary
 // element strides for rows, columns and the batch index (0 broadcasts), so
 // a (D, D, Nt) propagator contracts with a block of vectors without any
-// transposition.  FP64 on the tiled GEMM of gemm_f64.cuh (64 x 64 tiles).
+// transposition.  FP64 on the tiled GEMM of gemm_f64.cuh (64 x 64 tiles), or
+// one thread an element for outputs that would leave most of a tile empty;
+// both add the K terms of an element in the same order.
 
 #include "gemm_f64.cuh"
 
@@ -46,6 +48,31 @@ __global__ void __launch_bounds__(rf::kThreads) zgemm_kernel(Args a) {
   rf::gemm_tile(a.M, a.N, a.K, blockIdx.y * rf::kTile, blockIdx.x * rf::kTile, la, lb, epi);
 }
 
+// One thread an element, its operands through L1.  The FP64 pipe is the
+// bound in both kernels (4 K DFMA an element) and a tile computes its
+// padding: a 20 x 20 basis change of 100 states, 131 us on tiles, takes 10 us.
+__global__ void __launch_bounds__(128) zgemm_element_kernel(Args a, int64_t total) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+    const int j = (int)(e % a.N);
+    const int64_t zi = e / a.N;
+    const int i = (int)(zi % a.M);
+    const int64_t z = zi / a.M;
+    const double2* A = a.A + z * a.a_bs + (int64_t)i * a.a_rs;
+    const double2* B = a.B + z * a.b_bs + (int64_t)j * a.b_cs;
+    const double2* S = a.S ? a.S + z * a.s_bs : nullptr;
+    double2 acc = cz();
+#pragma unroll 4
+    for (int k = 0; k < a.K; ++k) {
+      double2 x = A[(int64_t)k * a.a_cs], y = B[(int64_t)k * a.b_rs];
+      if (a.conj_a) x.y = -x.y;
+      if (S != nullptr) x = cmul(x, S[(int64_t)k * a.s_ks]);
+      if (a.conj_b) y.y = -y.y;
+      cfma(acc, x, y);
+    }
+    a.C[z * a.c_bs + (int64_t)i * a.c_rs + (int64_t)j * a.c_cs] = acc;
+  }
+}
+
 }  // namespace zg
 }  // namespace lime
 
@@ -66,6 +93,17 @@ extern "C" int lime_zgemm_strided_f64(const LimeZgemmDesc* d, void* stream) {
   const unsigned gx = (unsigned)((d->N + rf::kTile - 1) / rf::kTile);
   const unsigned gy = (unsigned)((d->M + rf::kTile - 1) / rf::kTile);
   if (gy > 65535u) return LIME_ERR_UNSUPPORTED;
+  // elements: while the tiles hold more than twice the outputs, or leave
+  // most SMs without one (fewer than 76 tiles: an SM's share of elements is
+  // then the smaller)
+  const int64_t outputs = (int64_t)d->M * d->N * d->batch, tiles = (int64_t)gx * gy * d->batch;
+  if (tiles * rf::kTile * rf::kTile > 2 * outputs || tiles < 76) {
+    const int64_t blocks = (outputs + 127) / 128;
+    zg::zgemm_element_kernel<<<(unsigned)(blocks < 1 << 20 ? blocks : 1 << 20), 128, 0, st>>>(a, outputs);
+    LIME_CUDA_TRY(cudaGetLastError());
+    count_launch();
+    return LIME_OK;
+  }
   int64_t launches = 0;
   for (int z0 = 0; z0 < d->batch; z0 += 65535) {
     a.z0 = z0;
