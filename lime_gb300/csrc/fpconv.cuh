@@ -14,6 +14,8 @@
 //                         instructions
 //   widen_f32(x)          (double) x, exact; subnormal inputs through the
 //                         conversion instruction
+//   split_a(x, v0, h1, h2) x = 64 k + two fp16 residuals (|k| <= 127), the
+//                         entries of the A operands, for |x| < 2^13
 //   scale_pow2(d, e)      d * 2^e for a double whose result stays normal
 //                         (exponent-field add), else d * 2^e in FP64
 //
@@ -21,6 +23,7 @@
 // the host's own conversions bit for bit.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -130,6 +133,51 @@ __host__ __device__ __forceinline__ double scale_pow2(double d, int e) {
 #endif
   }
   return from_bits64(u + ((uint64_t)(int64_t)e << 52));
+}
+
+// fp16 rounding h of s too near to a midpoint between two fp16 values for an
+// s that is off by half its last place and 2^-36 to decide
+__host__ __device__ __forceinline__ bool near_tie(float s, float h) {
+  const float p = fmaxf(from_bits32(bits32(s) & 0x7f800000u), 6.103515625e-05f);   // 2^e, at least 2^-14
+  return fabsf(fabsf(s - h) - p * 4.8828125e-04f) <= p * 1.1920928955078125e-07f + 2.9103830456733704e-11f;
+}
+
+constexpr double kA0Max = 127.0;
+
+// x = v0 (64 k, |k| <= 127) + h1 + h2 (fp16, round to nearest even) for |x| <
+// 2^13 and infinities and NaN as the FP64 instructions give it (a residual
+// that rounds to zero may have the other sign).  x enters as a float pair,
+// which leaves out at most 2^-49 |x|; where a rounding is too close to a
+// midpoint for that, the FP64 instructions decide.
+__host__ __device__ __forceinline__ void split_a(double x, float& v0, __half& h1, __half& h2) {
+  const uint64_t u = bits64(x);
+  const int E = (int)((u >> 52) & 0x7FF);
+  if (E < 1023 - 25) {   // under 2^-25: three zeros
+    v0 = (u >> 63) ? -0.f : 0.f;
+    h1 = __float2half_rn((u << 1) == 0 ? 0.f : v0);
+    h2 = h1;
+    return;
+  }
+  if (E < 1023 + 13) {
+    float hi, lo;
+    split_f64(x, hi, lo);
+    const float t = hi * 0.015625f, k = rintf(t);
+    v0 = fminf(fmaxf(k, -(float)kA0Max), (float)kA0Max) * 64.f;
+    const float r = hi - v0;                     // exact: both multiples of hi's last place
+    const float s = r + lo;
+    const float bb = s - r;
+    const float e = (r - (s - bb)) + (lo - bb);  // r + lo = s + e
+    h1 = __float2half_rn(s);
+    const float h = __half2float(h1);
+    const float s2 = (s - h) + e;
+    h2 = __float2half_rn(s2);
+    if (fabsf(t - k) != 0.5f && !near_tie(s, h) && !near_tie(s2, __half2float(h2))) return;
+  }
+  const double kq = fmin(fmax(rint(x * (1.0 / 64.0)), -kA0Max), kA0Max);
+  const double r1 = x - kq * 64.0;
+  v0 = (float)(kq * 64.0);
+  h1 = __double2half(r1);
+  h2 = __double2half(r1 - (double)__half2float(h1));
 }
 
 }  // namespace fpconv

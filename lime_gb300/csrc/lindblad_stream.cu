@@ -896,6 +896,12 @@ extern "C" size_t lime_lindblad_stream_workspace(int32_t n, int32_t batch, int32
 
 namespace {
 
+// threads of convert_kernel: one per eight entries of its longest row, up to 256
+int lsm_convert_threads(const LsmLayout& l) {
+  const int t = (l.KC1 > l.KC2 ? l.KC1 : l.KC2) * sg::kCK / 8;
+  return t >= 256 ? 256 : (t + 31) / 32 * 32;
+}
+
 // The buffers of one streaming propagation inside its workspace.
 struct LsmRun {
   lsm::Args a;
@@ -976,7 +982,7 @@ int lsm_prepare(const LimeLindbladStreamDesc* d, LsmRun& r, cudaStream_t st, int
   r.heff_t = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(d->workspace) + L.total);
 
   const int per_g = L.MT1 * 128 + (K > 0 ? L.MT2 * 128 : 0);
-  lsm::convert_kernel<<<G * per_g, 256, 0, st>>>(reinterpret_cast<const double2*>(d->heff), d->heff_stride,
+  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(reinterpret_cast<const double2*>(d->heff), d->heff_stride,
                                                   reinterpret_cast<const double2*>(d->l_ops), d->l_stride, a, co, 0);
   LIME_CUDA_TRY(cudaGetLastError());
   ++launches;
@@ -1054,7 +1060,7 @@ extern "C" int lime_lindblad_rk4_stream(const LimeLindbladStreamDesc* d, void* s
                                              reinterpret_cast<const double2*>(d->drive_ops),
                                              d->drive_coef + (size_t)step * d->n_drive, d->n_drive, r.heff_t);
       LIME_CUDA_TRY(cudaGetLastError());
-      lsm::convert_kernel<<<G * L.np, 256, 0, st>>>(r.heff_t, G == 1 ? 0 : (int64_t)d->n * d->n, nullptr, 0, a,
+      lsm::convert_kernel<<<G * L.np, lsm_convert_threads(L), 0, st>>>(r.heff_t, G == 1 ? 0 : (int64_t)d->n * d->n, nullptr, 0, a,
                                                     r.co, 1);
       LIME_CUDA_TRY(cudaGetLastError());
       launches += 2;
@@ -1277,10 +1283,10 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
   int64_t launches = 0;
 
   const int per_g = L.MT1 * 128;
-  lsm::convert_kernel<<<G * per_g, 256, 0, st>>>(reinterpret_cast<const double2*>(d->heff), d->heff_stride,
+  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(reinterpret_cast<const double2*>(d->heff), d->heff_stride,
                                                   nullptr, 0, af, cf, 0);
   LIME_CUDA_TRY(cudaGetLastError());
-  lsm::convert_kernel<<<G * per_g, 256, 0, st>>>(reinterpret_cast<const double2*>(d->heff_adj),
+  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(reinterpret_cast<const double2*>(d->heff_adj),
                                                   d->heff_adj_stride, nullptr, 0, aa, ca, 0);
   LIME_CUDA_TRY(cudaGetLastError());
   launches += 2;
