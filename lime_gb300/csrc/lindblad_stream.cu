@@ -539,8 +539,7 @@ __global__ void init_kernel(Args a, const double2* rho, int batch) {
         const double2 z = rho[((size_t)b * a.n + y + i) * a.n + x];
         v = im ? z.y : z.x;
       }
-      hv[i] = (float)v;
-      lv[i] = (float)(v - (double)hv[i]);
+      fpconv::split_f64(v, hv[i], lv[i]);
       sv[i] = __fmul_rn(hv[i], a.sb);
       range |= !(fabsf(sv[i]) <= sg::kBMax);
     }
@@ -554,31 +553,69 @@ __global__ void init_kernel(Args a, const double2* rho, int batch) {
   if (range) atomicOr(a.status, LIME_FLAG_RANGE);
 }
 
-// obs[b][slot][o] = Tr(E_o rho_b) = sum_xy E_o[x][y] rho[y][x], fp64 from hi + lo;
-// diag: E holds only the diagonals E_o[x][x] ([P|1][n_obs][n]), n terms
-__global__ void observe_kernel(Args a, const double2* E, int64_t e_stride, int n_obs, double2* out, int n_slots,
-                               int slot, int diag) {
+// obs[b][slot][o] = Tr(E_o rho_b) = sum_xy E_o[x][y] rho[y][x], fp64 from hi + lo.
+// Only the nonzero entries cost FP64 work (projectors and dipoles are
+// sparse; a zero entry adds exactly zero, and non-finite states are flagged
+// by the stage kernels), so the time is the latency of reading E: a block of
+// 256 threads keeps 8 loads a thread in flight, 128 threads with one each
+// took 108 us for 64 dense 129 x 129 observables.
+constexpr int kObsThreads = 256;
+__device__ __forceinline__ double2 rho_at(const Args& a, size_t base, int x, int y) {
+  const size_t er = base + (size_t)x * a.np + y, ei = base + (size_t)(a.np + x) * a.np + y;
+  return make_double2(fpconv::widen_f32(a.Phi[er]) + fpconv::widen_f32(a.Plo[er]),
+                      fpconv::widen_f32(a.Phi[ei]) + fpconv::widen_f32(a.Plo[ei]));
+}
+__device__ __forceinline__ void add_term(double& sr, double& si, double2 e, double2 p) {
+  sr += e.x * p.x - e.y * p.y;
+  si += e.x * p.y + e.y * p.x;
+}
+__global__ void __launch_bounds__(kObsThreads) observe_kernel(Args a, const double2* E, int64_t e_stride, int n_obs,
+                                                              double2* out, int n_slots, int slot) {
   const int b = blockIdx.x / n_obs, o = blockIdx.x % n_obs;
-  const int per = diag ? a.n : a.n * a.n;
+  const int per = a.n * a.n;
   const double2* Eo = E + (e_stride ? (int64_t)(b % a.P) * e_stride : 0) + (int64_t)o * per;
   const size_t base = (size_t)b * inst_floats(a);
   double sr = 0.0, si = 0.0;
-  for (int q = threadIdx.x; q < per; q += blockDim.x) {
-    const int x = diag ? q : q / a.n, y = diag ? q : q - x * a.n;
-    const double2 ev = Eo[q];
-    // a zero entry adds exactly zero (projectors and dipoles are sparse);
-    // non-finite states are flagged by the stage kernels
-    if (ev.x == 0.0 && ev.y == 0.0) continue;
-    const size_t er = base + (size_t)x * a.np + y, ei = base + (size_t)(a.np + x) * a.np + y;
-    const double pr = (double)a.Phi[er] + (double)a.Plo[er];
-    const double pi = (double)a.Phi[ei] + (double)a.Plo[ei];
-    sr += ev.x * pr - ev.y * pi;
-    si += ev.x * pi + ev.y * pr;
+  constexpr int kN = 8;
+  for (int q0 = threadIdx.x; q0 < per; q0 += kN * kObsThreads) {
+    double2 ev[kN];
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      const int q = q0 + i * kObsThreads;
+      ev[i] = q < per ? Eo[q] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      if (ev[i].x == 0.0 && ev[i].y == 0.0) continue;
+      const int q = q0 + i * kObsThreads, x = q / a.n;
+      add_term(sr, si, ev[i], rho_at(a, base, x, q - x * a.n));
+    }
   }
   __shared__ double red[32];
-  sr = block_sum<128>(sr, red);
-  si = block_sum<128>(si, red);
+  sr = block_sum<kObsThreads>(sr, red);
+  si = block_sum<kObsThreads>(si, red);
   if (threadIdx.x == 0) out[((size_t)b * n_slots + slot) * n_obs + o] = make_double2(sr, si);
+}
+
+// The same for diagonal observables, E holding their diagonals
+// ([P|1][n_obs][n]): a warp each.
+__global__ void __launch_bounds__(128) observe_diag_kernel(Args a, const double2* E, int64_t e_stride, int n_obs,
+                                                           int batch, double2* out, int n_slots, int slot) {
+  const int64_t w = blockIdx.x * (int64_t)4 + (threadIdx.x >> 5);
+  const int b = (int)(w / n_obs), o = (int)(w % n_obs), lane = threadIdx.x & 31;
+  if (b >= batch) return;
+  const double2* Eo = E + (e_stride ? (int64_t)(b % a.P) * e_stride : 0) + (int64_t)o * a.n;
+  const size_t base = (size_t)b * inst_floats(a);
+  double sr = 0.0, si = 0.0;
+  for (int x = lane; x < a.n; x += 32) {
+    const double2 ev = Eo[x];
+    if (ev.x != 0.0 || ev.y != 0.0) add_term(sr, si, ev, rho_at(a, base, x, x));
+  }
+  for (int k = 16; k > 0; k >>= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, k);
+    si += __shfl_xor_sync(0xffffffffu, si, k);
+  }
+  if (lane == 0) out[((size_t)b * n_slots + slot) * n_obs + o] = make_double2(sr, si);
 }
 
 __global__ void final_kernel(Args a, double2* rho, int batch) {
@@ -587,9 +624,7 @@ __global__ void final_kernel(Args a, double2* rho, int batch) {
     const int b = (int)(q / ((size_t)a.n * a.n));
     const int rem = (int)(q % ((size_t)a.n * a.n));
     const int y = rem / a.n, x = rem - y * a.n;
-    const size_t base = (size_t)b * inst_floats(a);
-    const size_t er = base + (size_t)x * a.np + y, ei = base + (size_t)(a.np + x) * a.np + y;
-    rho[q] = make_double2((double)a.Phi[er] + (double)a.Plo[er], (double)a.Phi[ei] + (double)a.Plo[ei]);
+    rho[q] = rho_at(a, (size_t)b * inst_floats(a), x, y);
   }
 }
 
@@ -781,11 +816,11 @@ __global__ void __launch_bounds__(256) adj_finish_kernel(Args a, AdjState j, int
 //   d/dJ_k    += 2 sum_x Im(conj(ab_kx) y_k+1,x) + Im(conj(ab_k+1,x) y_kx)
 //   d/dgamma_k -= sum_{x != k} Re(conj(ab_kx) y_kx)
 // One block per (instance, run of 8 rows), threads over the columns.
-__global__ void adj_grad_kernel(Args a, const float* ab, const float* yst, int batch, double* gd, double* gb,
-                                double* gg) {
-  const int runs = a.np / 8;
+constexpr int kGradThreads = 128;
+__global__ void __launch_bounds__(kGradThreads) adj_grad_kernel(Args a, const float* ab, const float* yst, double* gd,
+                                                                double* gb, double* gg) {
+  const int runs = (a.n + 7) / 8;
   const int b = blockIdx.x / runs, k0 = (blockIdx.x % runs) * 8;
-  if (b >= batch || k0 >= a.n) return;
   const int n = a.n, np = a.np;
   const float* A = ab + (size_t)b * inst_floats(a);
   const float* Y = yst + (size_t)b * inst_floats(a);
@@ -797,15 +832,17 @@ __global__ void adj_grad_kernel(Args a, const float* ab, const float* yst, int b
   for (int i = 0; i < 24; ++i) pf[i] = 0.f;
   for (int x = threadIdx.x; x < n; x += blockDim.x) {
     float ar[9], ai[9], yr[9], yi[9];
+    const auto load = [&](const float* p, float (&v)[9]) {
+      float w[8];
+      sg::ld8(p, w);
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const int k = k0 + i;
-      const bool ok = k < np;
-      ar[i] = ok ? A[(size_t)x * np + k] : 0.f;
-      ai[i] = ok ? A[(size_t)(np + x) * np + k] : 0.f;
-      yr[i] = ok ? Y[(size_t)x * np + k] : 0.f;
-      yi[i] = ok ? Y[(size_t)(np + x) * np + k] : 0.f;
-    }
+      for (int i = 0; i < 8; ++i) v[i] = w[i];
+      v[8] = k0 + 8 < np ? p[8] : 0.f;
+    };
+    load(A + (size_t)x * np + k0, ar);
+    load(A + (size_t)(np + x) * np + k0, ai);
+    load(Y + (size_t)x * np + k0, yr);
+    load(Y + (size_t)(np + x) * np + k0, yi);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int k = k0 + i;
@@ -818,22 +855,20 @@ __global__ void adj_grad_kernel(Args a, const float* ab, const float* yst, int b
       }
     }
   }
-  double part[24];
+  // the block's sums in fp64, four threads a sum: 24 shuffle trees of doubles
+  // a warp were 480 FP64 instructions a block, this is 99
+  __shared__ float red[24][kGradThreads + 1];
 #pragma unroll
-  for (int i = 0; i < 24; ++i) part[i] = (double)pf[i];
-  __shared__ double red[4][24];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-#pragma unroll
-  for (int i = 0; i < 24; ++i) {
-    double v = part[i];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (l == 0) red[w][i] = v;
-  }
+  for (int i = 0; i < 24; ++i) red[i][threadIdx.x] = pf[i];
   __syncthreads();
-  if (threadIdx.x < 24) {
-    const int i = threadIdx.x;
-    double v = 0.0;
-    for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) v += red[ww][i];
+  double v = 0.0;
+  const int cols = n < kGradThreads ? n : kGradThreads;
+  if (threadIdx.x < 96)
+    for (int t = threadIdx.x & 3; t < cols; t += 4) v += fpconv::widen_f32(red[threadIdx.x >> 2][t]);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  if (threadIdx.x < 96 && (threadIdx.x & 3) == 0) {
+    const int i = threadIdx.x >> 2;
     const int k = k0 + (i & 7);
     const int nb = n > 1 ? n - 1 : 1;
     if (k < n) {
@@ -1015,11 +1050,15 @@ void lsm_bind_stage(LsmRun& r, int s, int cur) {
 int lsm_observe(const LimeLindbladStreamDesc* d, LsmRun& r, int step, cudaStream_t st, int64_t& launches) {
   const int obs_every = d->obs_every > 0 ? d->obs_every : 1;
   if (d->n_obs > 0 && ((step + 1) % obs_every) == 0) {
-    lsm::observe_kernel<<<r.B * d->n_obs, 128, 0, st>>>(r.a, reinterpret_cast<const double2*>(d->obs_ops),
-                                                        d->obs_stride, d->n_obs,
-                                                        reinterpret_cast<double2*>(d->obs_out),
-                                                        d->n_steps / obs_every, (step + 1) / obs_every - 1,
-                                                        d->obs_diag);
+    const double2* E = reinterpret_cast<const double2*>(d->obs_ops);
+    double2* out = reinterpret_cast<double2*>(d->obs_out);
+    const int slots = d->n_steps / obs_every, slot = (step + 1) / obs_every - 1;
+    if (d->obs_diag)
+      lsm::observe_diag_kernel<<<(unsigned)(((int64_t)r.B * d->n_obs + 3) / 4), 128, 0, st>>>(
+          r.a, E, d->obs_stride, d->n_obs, r.B, out, slots, slot);
+    else
+      lsm::observe_kernel<<<r.B * d->n_obs, lsm::kObsThreads, 0, st>>>(r.a, E, d->obs_stride, d->n_obs, out, slots,
+                                                                       slot);
     LIME_CUDA_TRY(cudaGetLastError());
     ++launches;
   }
@@ -1354,8 +1393,8 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
         aa.Sn = Sbuf[c ^ 1];
         lsm::gemm_kernel<false><<<gemm_grid, sg::kThreads, smem, st>>>(aa);
         LIME_CUDA_TRY(cudaGetLastError());
-        lsm::adj_grad_kernel<<<B * (L.np / 8), 128, 0, st>>>(aa, Sbuf[c], store + ((size_t)s * 4 + (i - 1)) * B * inst,
-                                                             B, d->grad_diag, d->grad_bond, d->grad_gamma);
+        lsm::adj_grad_kernel<<<B * ((d->n + 7) / 8), lsm::kGradThreads, 0, st>>>(
+            aa, Sbuf[c], store + ((size_t)s * 4 + (i - 1)) * B * inst, d->grad_diag, d->grad_bond, d->grad_gamma);
         LIME_CUDA_TRY(cudaGetLastError());
         const float c_l = (float)(i == 2 ? dt / 6.0 : dt / 3.0);
         const float c_y = (float)(i == 4 ? dt : dt / 2.0);
