@@ -49,6 +49,15 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
+def _host_or_device(a, device):
+    """A host operator as a dense complex128 array, a device tensor on ``device``."""
+    if isinstance(a, torch.Tensor) and a.device.type != 'cpu':
+        return as_device(a, device)
+    if isinstance(a, torch.Tensor):
+        a = a.detach().resolve_conj()
+    return np.asarray(_to_dense_np(a), dtype=np.complex128)
+
+
 class DiagonalOps:
     """K diagonal collapse operators given by their diagonals.
 
@@ -116,10 +125,15 @@ def expand_e_ops(e_ops, n: int):
     return e_ops
 
 
-def is_diagonal(op: torch.Tensor) -> bool:
+def _off_diagonal(op: torch.Tensor) -> torch.Tensor:
+    """Number of nonzero off-diagonal entries, on the device."""
     n = op.shape[-1]
     off = op * (1 - torch.eye(n, dtype=op.dtype, device=op.device))
-    return bool(torch.count_nonzero(off) == 0)
+    return torch.count_nonzero(off)
+
+
+def is_diagonal(op: torch.Tensor) -> bool:
+    return bool(_off_diagonal(op) == 0)
 
 
 @dataclass
@@ -155,7 +169,7 @@ class LindbladGenerator:
         rates = [c.rates_on(device) for c in c_ops if isinstance(c, SiteDephasing)]
         c_ops = [c for c in c_ops if not isinstance(c, SiteDephasing)]
         packed = [as_device(c.l, device) for c in c_ops if isinstance(c, DiagonalOps)]
-        ops = [as_device(c, device) for c in c_ops if not isinstance(c, DiagonalOps)]
+        ops = [_host_or_device(c, device) for c in c_ops if not isinstance(c, DiagonalOps)]
         P = Hd.shape[0]
         for r in rates:
             if r.shape[-1] != n:
@@ -175,25 +189,35 @@ class LindbladGenerator:
             if c.shape[-2:] != (n, n):
                 raise ValueError('collapse operator shape %s does not match H (%d, %d)'
                                  % (tuple(c.shape), n, n))
-            if c.dim() == 3:
+            if c.ndim == 3:
                 if P not in (1, c.shape[0]):
                     raise ValueError('inconsistent batch sizes in H and c_ops')
                 P = c.shape[0]
         shared = (P == 1)
-        diag = [c for c in ops if is_diagonal(c)]
-        dense = [c for c in ops if not is_diagonal(c)]
+        # host operators are sorted on the host: a test on the device is a
+        # handful of launches and a read back for each operator
+        kinds = [is_diagonal(c) if isinstance(c, torch.Tensor) else _is_diag_host(c) for c in ops]
+        diag = [c for c, k in zip(ops, kinds) if k]
+        dense = [c for c, k in zip(ops, kinds) if not k]
 
         def stack(lst, per):
-            # -> (P|1, K, ...) with per-instance broadcast when mixed
+            # -> (P|1, K, ...) with per-instance broadcast when mixed; shared host operators in one upload
             if not lst:
                 return None
+            if not any(isinstance(x, torch.Tensor) for x in lst) and all(x.ndim == per for x in lst):
+                return as_device(np.stack(lst)[None], device)
+            lst = [as_device(x, device) for x in lst]
             if all(x.dim() == per for x in lst):
                 return torch.stack(lst, 0).unsqueeze(0).contiguous()
             return torch.stack([x.expand((P,) + x.shape[-per:]) if x.dim() == per else x
                                 for x in lst], 1).contiguous()
 
         ld = stack(dense, 2)
-        lg = stack([torch.diagonal(x, dim1=-2, dim2=-1) for x in diag], 1)
+        lg = stack([torch.diagonal(x, dim1=-2, dim2=-1) if isinstance(x, torch.Tensor) else
+                    np.diagonal(x, axis1=-2, axis2=-1) for x in diag], 1)
+        # operators |k><k| (times a factor) give a diagonal M
+        m_diagonal = not packed and all(not isinstance(x, torch.Tensor) and
+                                        np.count_nonzero(x, axis=(-2, -1)).max(initial=0) <= 1 for x in diag)
         if packed:
             parts = ([] if lg is None else [lg]) + [p if p.dim() == 3 else p.unsqueeze(0) for p in packed]
             if any(x.shape[0] != 1 for x in parts):
@@ -223,8 +247,8 @@ class LindbladGenerator:
         nat.check(lib.lime_lindblad_prepare_f64(d, _stream_ptr()), 'lime_lindblad_prepare_f64')
         gen = LindbladGenerator(n=n, P=P, heff=heff, m=(m if lg is not None or rate is not None else None),
                                 l_dense=ld, k_dense=d.k_dense, shared=shared)
-        if lg is None and rate is not None:
-            gen.split_cache['m_diagonal'] = True   # site dephasing alone: M = diag(rates)
+        if gen.m is not None and m_diagonal:
+            gen.split_cache['m_diagonal'] = True   # M = diag(rates), or one entry an operator
         return gen
 
 
@@ -247,7 +271,14 @@ def prepare_obs(e_ops, n, P, device):
         return Et, e_ops.count, 1, 0
     if not e_ops:
         return None, 0, 0, 0
-    E = [as_device(e, device) for e in e_ops]
+    E = [_host_or_device(e, device) for e in e_ops]
+    if all(not isinstance(e, torch.Tensor) and e.shape == (n, n) for e in E):
+        # host operators: inspected on the host, one upload
+        Eh = np.stack(E)
+        if _is_diag_host(Eh):
+            return as_device(np.diagonal(Eh, axis1=-2, axis2=-1)[None].copy(), device), len(E), 1, 0
+        return as_device(Eh[None], device), len(E), 0, 0
+    E = [as_device(e, device) for e in E]
     per = any(e.dim() == 3 for e in E)
     if per:
         E = [e.expand(P, n, n) if e.dim() == 2 else e for e in E]
@@ -320,10 +351,18 @@ def split_supported(gen: LindbladGenerator) -> str | None:
             why = 'dimension %d > %d' % (gen.n, SPLIT_MAX_N)
         elif gen.k_dense:
             why = 'dense (non-diagonal) collapse operators'
-        elif gen.m is not None and not c.get('m_diagonal') and not is_diagonal(gen.m):
+        elif gen.m is not None and not m_is_diagonal(gen):
             why = 'diagonal collapse operators with a non-diagonal M = sum_k l_k l_k^dag'
         c['why'] = why
     return c['why']
+
+
+def m_is_diagonal(gen: LindbladGenerator) -> bool:
+    """Whether M is diagonal (decided once per generator)."""
+    c = gen.split_cache
+    if 'm_diagonal' not in c:
+        c['m_diagonal'] = is_diagonal(gen.m)
+    return c['m_diagonal']
 
 
 def _pow2_exponent(target: float, bound: float) -> int:
@@ -369,8 +408,9 @@ def _is_diag_host(a) -> bool:
     if a.ndim < 2 or a.shape[-1] != a.shape[-2]:
         return False
     n = a.shape[-1]
-    m = a.reshape(-1, n, n)
-    return not np.any(m[:, ~np.eye(n, dtype=bool)])
+    m = a.reshape(-1, n * n)
+    # the off-diagonal entries: all but every (n + 1)-th
+    return n < 2 or not np.any(m[:, :-1].reshape(-1, n - 1, n + 1)[:, :, 1:])
 
 
 def _host_array(a):
@@ -535,25 +575,33 @@ def _run_stream(gen: LindbladGenerator, rho: torch.Tensor, dt: float, n_steps: i
         else:
             E = torch.stack(Es, 0).unsqueeze(0).contiguous()
         n_obs = E.shape[1]
-        if not obs_diag and any(h is None for h in host):
-            # device operators: one check per call
-            obs_diag = bool(is_diagonal(E.reshape(-1, n, n)))
-        if obs_diag:
-            E = torch.diagonal(E, dim1=-2, dim2=-1).contiguous()
     n_slots = n_steps // obs_every
     obs_out = torch.zeros((B, max(n_slots, 1), max(n_obs, 1)), dtype=CDT, device=dev)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
-    pmax = float(torch.view_as_real(rho).abs().max().item()) if rho.numel() else 0.0
-    lrow = 0.0
-    if K:
-        lrow = float(gen.l_dense.abs().sum(-1).max().item())
+    # one read back: max |rho0|, the operators' largest absolute row sum (once
+    # per generator) and whether device observables are diagonal
+    facts = [torch.view_as_real(rho).abs().max() if rho.numel() else torch.zeros((), dtype=torch.float64, device=dev)]
+    if K and 'lrow' not in gen.split_cache:
+        facts.append(gen.l_dense.abs().sum(-1).max())
+    ask_diag = n_obs > 0 and not obs_diag and any(h is None for h in host)
+    if ask_diag:
+        facts.append(_off_diagonal(E).double())
+    facts = torch.stack(facts).tolist()
+    pmax = facts[0]
+    if K and 'lrow' not in gen.split_cache:
+        gen.split_cache['lrow'] = facts[1]
+    lrow = gen.split_cache['lrow'] if K else 0.0
+    if ask_diag:
+        obs_diag = facts[-1] == 0
+    if obs_diag:
+        E = torch.diagonal(E, dim1=-2, dim2=-1).contiguous()
     scales = [_pow2_exponent(8192.0 / 1.25, pmax), _pow2_exponent(8192.0 / 1.25, lrow * pmax) if K else 0]
     heff_shared = gen.heff.shape[0] == 1
     l_shared = gen.l_dense is None or gen.l_dense.shape[0] == 1
     # a diagonal M (pure dephasing) goes in as its real diagonal
     m_diag = None
-    if gen.m is not None and (gen.split_cache.get('m_diagonal') or is_diagonal(gen.m)):
-        m_diag = torch.diagonal(gen.m, dim1=-2, dim2=-1).real.contiguous()
+    if gen.m is not None and m_is_diagonal(gen):
+        m_diag = split_operands_mdiag(gen)
     G = 1 if (heff_shared and l_shared) else param_batch
     wsb = lib.lime_lindblad_stream_workspace(n, B, G, K)
     ws = torch.empty(wsb + 1024, dtype=torch.uint8, device=dev)
@@ -860,7 +908,7 @@ def propagate_host_pipelined(H, rho0, c_ops, e_ops, dt: float, n_steps: int, obs
         return None
     if not isinstance(e_ops, Populations) and e_ops and any(_ndim(e) != 2 for e in e_ops):
         return None
-    if not _host_hermitian(rho0):
+    if _host_array(rho0) is None:
         return None
     nat.require_device()
     comp = torch.cuda.current_stream(device)
@@ -926,7 +974,14 @@ def propagate_host_pipelined(H, rho0, c_ops, e_ops, dt: float, n_steps: int, obs
         finishers.append(fin)
     down.synchronize()
     for fin in finishers:
-        fin(True)                        # raises on a kernel status flag
+        try:
+            fin(True)                    # raises on a kernel status flag
+        except nat.KernelFlagError as err:
+            # the kernel compares every rho(0) with its adjoint (a pass over
+            # the batch on the host took longer than the whole pipeline)
+            if err.flags & nat.LIME_FLAG_NOT_HERMITIAN:
+                return None
+            raise
     del keep, inputs, gens, amax
     return obs_h, rho_h
 

@@ -29,9 +29,7 @@ def _as_tensor(f, device):
 
 def _freq(nx: int, dx: float) -> np.ndarray:
     """2 pi fftshift(fftfreq(nx, dx)) (numpy's layout)."""
-    k = np.arange(nx)
-    f = np.where(k < (nx + 1) // 2, k, k - nx) / (nx * dx)
-    return 2.0 * math.pi * np.roll(f, nx // 2)
+    return 2.0 * math.pi * ((np.arange(nx) - nx // 2) / (nx * dx))
 
 
 def _dft_rows(x: torch.Tensor, inverse: bool, shift: bool, post: torch.Tensor | None) -> torch.Tensor:
@@ -84,14 +82,19 @@ def fft(f, x=None, axis=-1, device=None):
         x = np.arange(nx)
     x = np.asarray(x.detach().cpu() if isinstance(x, torch.Tensor) else x, dtype=np.float64)
     dx = float(x[1] - x[0])
-    freq = _freq(nx, dx)
-    post = torch.as_tensor(dx * np.exp(-1j * freq * float(x[0])), dtype=CDT, device=dev)
+    # one upload: the factors dx exp(-i w x0), then the grid
+    host = np.empty(3 * nx)
+    host[2 * nx:] = freq = _freq(nx, dx)
+    arg = freq * float(x[0])
+    host[0:2 * nx:2] = dx * np.cos(arg)
+    host[1:2 * nx:2] = -dx * np.sin(arg)
+    both = torch.as_tensor(host, device=dev)
+    post = torch.view_as_complex(both[:2 * nx].reshape(nx, 2))
     moved = ft.movedim(axis, -1)
     lead = moved.shape[:-1]
     g = _Spectrum.apply(moved.reshape(-1, nx), post).reshape(lead + (nx,)).movedim(-1, axis)
-    fr = torch.as_tensor(freq, dtype=torch.float64, device=dev)
     if is_t:
-        return g, fr
+        return g, both[2 * nx:].clone()
     return g.detach().cpu().numpy(), freq
 
 
