@@ -214,7 +214,7 @@ class LindbladGenerator:
 
         ld = stack(dense, 2)
         lg = stack([torch.diagonal(x, dim1=-2, dim2=-1) if isinstance(x, torch.Tensor) else
-                    np.diagonal(x, axis1=-2, axis2=-1) for x in diag], 1)
+                    np.diagonal(x, axis1=-2, axis2=-1).copy() for x in diag], 1)
         # operators |k><k| (times a factor) give a diagonal M
         m_diagonal = not packed and all(not isinstance(x, torch.Tensor) and
                                         np.count_nonzero(x, axis=(-2, -1)).max(initial=0) <= 1 for x in diag)
