@@ -133,6 +133,7 @@ struct Args {
   size_t rho_elems = kNoExtent, obs_elems = kNoExtent, a_words = kNoExtent;
 };
 
+template <int kWarps = kThreads / 32>
 __device__ __forceinline__ double block_sum(double v, double* red, int t) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -141,7 +142,7 @@ __device__ __forceinline__ double block_sum(double v, double* red, int t) {
   __syncthreads();
   double s = 0.0;
 #pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) s += red[w];
+  for (int w = 0; w < kWarps; ++w) s += red[w];
   return s;
 }
 
@@ -171,7 +172,8 @@ __device__ __forceinline__ float row_magic(float m) {
 }
 
 // Split 8 consecutive B^T values into b0 (q grid) + b1 (fp16 residual) and store.
-__device__ __forceinline__ void store_b8(Smem& S, uint32_t off, const float* x, float magic, float& mx) {
+template <class SmemT>
+__device__ __forceinline__ void store_b8(SmemT& S, uint32_t off, const float* x, float magic, float& mx) {
   uint32_t h0[4], h1[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -869,6 +871,483 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
   }
 }
 
+// ---------------------------------------------------------------- n <= 32
+// The same propagation for dimensions up to kW = 16 or 32, without the work
+// of the padding to 64: N = kW columns, the 2 kW entries of K that a row has,
+// and 64 rows in 128 threads.  The [Xr; Xi] rows are laid out as
+//     lanes 32 q ..: q = 0, 1 Xr, q = 2, 3 Xi   (row i = lane & 31, both copies)
+// so that warp q takes columns [kW/2 (q & 1), + kW/2) of its component in its
+// own TMEM quadrant and all four warps work.  The sums are those of the
+// 64-wide kernel bit for bit: the left-out products are exact zeros, K runs
+// through the same groups of 16 in the same order, and the fp32 sums over a
+// row (the norm that sets the B scale, dense observables) are chained in
+// its column order.
+// kDual: the small products and the exact one accumulate in columns of their
+// own, so a stage has one MMA wait instead of two; it takes twice the tensor
+// memory of the kW = 32 form (kCtas).
+//
+// Bound: a stage's chain of MMA, TMEM load, transpose and B store (one
+// instance), the issue slots of the epilogue (batches).  Measured against the
+// 64-wide kernel: 4096 instances, 20 steps, n = 16: 4.66 -> 0.72 ms, n = 32:
+// 4.70 -> 1.40 ms; one 16-site chain 3.1 -> 1.0 us a stage.
+template <int kW>
+struct __align__(128) SmallSmem {
+  uint8_t bop[2][4 * kW * kW];           // B0, B1: kW (N) x 2 kW (K) fp16
+  float xt[2 * kW * (kW + 4)];           // D transpose buffer, row = component * kW + i
+  float rlo[kW / 2 * 128];               // compensation of rho, [j][t]
+  float smax[2][128];
+  float obsp[2][128];                    // dense observables: partial sums of the first column half
+  double red[2][4];
+  float redf[4];
+  double trp[2], trs[2], tr0;
+  int eb;
+  uint64_t mbar;
+  uint32_t tmem_base;
+};
+
+template <int kW, bool kDual>
+struct SmallShape {
+  static constexpr int kThreads = 128;
+  static constexpr int kHalf = kW / 2;                                  // columns of a thread
+  static constexpr uint32_t kD = 3 * kW, kD1 = kDual ? 4 * kW : 3 * kW;  // exact product, small products
+  static constexpr uint32_t kUsed = kD1 + kW;
+  static constexpr uint32_t kTmem = kUsed <= 64 ? 64 : kUsed <= 128 ? 128 : 256;
+  static constexpr int kCtas = 512 / kTmem;                             // resident CTAs per SM
+  static_assert(kW == 16 || kW == 32, "whole K groups of 16, a row per lane");
+  static_assert(2 * sizeof(SmallSmem<kW>::bop[0]) + sizeof(SmallSmem<kW>::xt) >= kW * kW * 16 &&
+                    offsetof(SmallSmem<kW>, xt) == 2 * sizeof(SmallSmem<kW>::bop[0]),
+                "the staged kW x kW complex128 matrix fits the B and transpose buffers");
+};
+
+// columns [col, col + kC) of a thread's TMEM lane
+template <int kC>
+__device__ __forceinline__ void tmem_ld(uint32_t addr, float (&v)[kC]) {
+  uint32_t r[kC / 8][8];
+#pragma unroll
+  for (int c = 0; c < kC / 8; ++c) tc::tmem_ld8_nowait(addr + 8 * c, r[c]);
+  tc::tmem_wait_ld();
+#pragma unroll
+  for (int c = 0; c < kC; ++c) v[c] = __uint_as_float(r[c / 8][c % 8]);
+}
+
+template <int kW, bool kDual>
+__device__ __forceinline__ void small_mma(uint32_t tbase, uint64_t desc_b0, uint64_t desc_b1, bool small, bool exact) {
+  using Sh = SmallShape<kW, kDual>;
+  constexpr uint32_t idesc = tc::idesc_f16(128, kW, 0);
+#pragma unroll
+  for (int ks = 0; ks < kW / 8; ++ks) {
+    const uint64_t d0 = desc_b0 + (uint64_t)(2 * kLBO / 16) * ks, d1 = desc_b1 + (uint64_t)(2 * kLBO / 16) * ks;
+    const uint32_t acc = ks > 0 ? 1u : 0u, a = tbase + 8 * ks;
+    if (small) {
+      tc::mma_f16_ts(tbase + Sh::kD1, a + kW, d0, idesc, acc);
+      tc::mma_f16_ts(tbase + Sh::kD1, a, d1, idesc, 1u);
+      tc::mma_f16_ts(tbase + Sh::kD1, a + kW, d1, idesc, 1u);
+      tc::mma_f16_ts(tbase + Sh::kD1, a + 2 * kW, d0, idesc, 1u);
+    }
+    if (exact) tc::mma_f16_ts(tbase + Sh::kD, a, d0, idesc, acc);
+  }
+}
+
+template <int kW, bool kDual>
+__global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_rk4_split_small_kernel(Args a) {
+  using Sh = SmallShape<kW, kDual>;
+  constexpr int kC = Sh::kHalf, kLd = kW + 4;
+  constexpr uint32_t kS = 32 * kW;         // B operand: N-direction 8-row-group stride (bytes)
+  extern __shared__ uint8_t smem_raw[];
+  SmallSmem<kW>& S =
+      *reinterpret_cast<SmallSmem<kW>*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  const int t = threadIdx.x, q = t >> 5, i = t & 31;
+  const bool is_re = q >= 2, on = i < kW;
+  const int h = q & 1, j0 = kC * h;
+  const int row = (is_re ? kW : 0) + i;            // of the transpose buffer
+  const bool diag_owner = is_re && on && i / kC == h;
+  const int n = a.n;
+
+  if (q == 0) {
+    tc::tmem_alloc(&S.tmem_base, Sh::kTmem);
+    tc::tmem_relinquish();
+  }
+  if (t == 0) {
+    tc::mbar_init(&S.mbar, 1);
+    tc::mbar_fence_init();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tbase = S.tmem_base;
+  const uint32_t lane_addr = tbase + ((uint32_t)(q * 32) << 16);
+  const uint64_t desc_b0 = tc::smem_desc_noswizzle(tc::smem_u32(S.bop[0]), kLBO, kS);
+  const uint64_t desc_b1 = tc::smem_desc_noswizzle(tc::smem_u32(S.bop[1]), kLBO, kS);
+  const uint32_t bseg = (uint32_t)(i >> 3) * kS + (uint32_t)(i & 7) * 16u +
+                        ((is_re ? 0u : (uint32_t)kW / 8) + (uint32_t)(kC / 8 * h)) * kLBO;
+  const float tsign = is_re ? 1.f : -1.f;
+  float* xrow = S.xt + (on ? row : 0) * kLd;
+  const float* xcol = S.xt + (is_re ? kW : 0) * kLd + (on ? i : 0);
+  auto at = [](int r, int c) { return r * kW + (c ^ (r & 7)); };   // staged element, as stage_index
+  uint32_t phase = 0;
+  int flags = 0;
+  bool aborted = false;
+  int g = 0;
+
+  for (int b = blockIdx.x; b < a.batch && !aborted; b += gridDim.x) {
+    const int p = b % a.param_batch;
+    const double2* heff = a.heff + p * a.heff_stride;
+    const float mi = (a.m_diag && i < n) ? (float)a.m_diag[p * a.m_stride + i] : 0.f;
+
+    // ---- A operand: K = [re kW | im kW], words [piece][component][kW / 2] ----
+    {
+      const int r64 = (is_re ? 64 : 0) + i;        // row of the prepared pieces
+      float magic = 0.f, qmax = 0.f;
+      if (!a.a_pieces) a_row_quantum(a_row_max(heff, n, i, is_re, a.sa_d), magic, qmax);
+#pragma unroll 1
+      for (int hh = 0; hh < 2; ++hh) {
+        uint32_t w[3][16];
+        if (a.a_pieces) {
+          const uint4* src = a.a_pieces + (int64_t)p * a.a_stride;
+#pragma unroll
+          for (int piece = 0; piece < 3; ++piece)
+#pragma unroll
+            for (int c4 = 0; c4 < kW / 8; ++c4) {
+              const int at4 = a_piece_index(piece, 0, hh, c4, r64);
+              const uint4 v = in_bounds(((size_t)p * a.a_stride + at4) * 16, 16, a.a_words * 16, a.status)
+                                  ? src[at4] : make_uint4(0, 0, 0, 0);
+              w[piece][4 * c4] = v.x; w[piece][4 * c4 + 1] = v.y;
+              w[piece][4 * c4 + 2] = v.z; w[piece][4 * c4 + 3] = v.w;
+            }
+        } else {
+          a_pieces_row(heff, n, i, is_re, hh, 0, a.sa_d, magic, qmax, w[0], w[1], w[2]);
+        }
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece)
+#pragma unroll
+          for (int c = 0; c < kW / 16; ++c) {
+            uint32_t v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = w[piece][8 * c + e];
+            tc::tmem_st8(lane_addr + (uint32_t)(piece * kW + hh * kC + 8 * c), v);
+          }
+      }
+      tc::tmem_wait_st();
+    }
+
+    // ---- state, staged as in the 64-wide kernel ----
+    double2* stg = reinterpret_cast<double2*>(S.bop[0]);
+    {
+      const double2* r0 = a.rho + (int64_t)b * n * n;
+      for (int e = t; e < kW * kW; e += Sh::kThreads) {
+        const int ii = e / kW, jj = e % kW;
+        double2 z = make_double2(0.0, 0.0);
+        if (ii < n && jj < n &&
+            in_bounds(((size_t)b * n * n + ii * n + jj) * 16, 16, a.rho_elems * 16, a.status))
+          z = r0[ii * n + jj];
+        stg[at(ii, jj)] = z;
+      }
+    }
+    __syncthreads();
+    float rho[kC], acc[kC];
+    double dtr = 0.0;
+    float fro = 0.f;
+    bool herm = true;
+    {
+      const double* sd = reinterpret_cast<const double*>(stg);
+      const int comp = is_re ? 0 : 1;
+      const uint64_t flip = is_re ? 0ull : 0x8000000000000000ull;
+#pragma unroll
+      for (int jj = 0; jj < kC; ++jj) {
+        const int j = j0 + jj;
+        float hv = 0.f, lv = 0.f;
+        if (on) {
+          const double v = sd[2 * at(i, j) + comp];
+          const uint64_t bv = fpconv::bits64(v);
+          const uint64_t bw = fpconv::bits64(sd[2 * at(j, i) + comp]) ^ flip;
+          herm &= (bv == bw) || ((bv | bw) << 1) == 0;
+          fpconv::split_f64(v, hv, lv);
+          if (diag_owner && j == i) dtr = v;
+        }
+        rho[jj] = hv;
+        acc[jj] = 0.f;
+        S.rlo[jj * 128 + t] = lv;
+      }
+      if (on && h == 0)
+        for (int j = 0; j < kW; ++j) {   // the whole row, in column order
+          float hv, lv;
+          fpconv::split_f64(sd[2 * at(i, j) + comp], hv, lv);
+          fro = __fmaf_rn(hv, hv, fro);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
+    if (is_re) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dtr += __shfl_xor_sync(0xffffffffu, dtr, o);
+      if (i == 0) S.trs[h] = dtr;
+    }
+    if (i == 0) S.redf[q] = fro;
+    __syncthreads();   // (also: every read of the staged matrix is done)
+    float fro_all = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) fro_all += S.redf[w];
+    int eb = a.eb;
+    if (a.auto_b) {
+      const float bound = sqrtf((float)n * fro_all);
+      eb = 0;
+      if (bound > 0.f && isfinite(bound)) {
+        const int e = ilogbf(bound);
+        eb = (bound == ldexpf(1.f, e)) ? 13 - e : 12 - e;
+        eb = max(-60, min(60, eb));
+      }
+    }
+    const float sbi = ldexpf(1.f, eb);
+    const float bsign = is_re ? sbi : -sbi;
+    float mx = 0.f;
+    float rho_d = 0.f, acc_d = 0.f, rs_d = 0.f;
+#pragma unroll
+    for (int jj = 0; jj < kC; ++jj) {
+      rho[jj] *= bsign;
+      S.rlo[jj * 128 + t] *= bsign;
+      mx = fmaxf(mx, fabsf(rho[jj]));
+      if (diag_owner && j0 + jj == i) rho_d = rho[jj];
+    }
+    if (!herm) flags |= LIME_FLAG_NOT_HERMITIAN;
+    rs_d = rho_d;
+    S.smax[g & 1][t] = mx;
+    if (t == 0) {
+      S.tr0 = S.trs[0] + S.trs[1];
+      S.eb = eb;
+    }
+    __syncthreads();
+    auto row_bound = [&]() {
+      const float* m = S.smax[g & 1];
+      return fmaxf(fmaxf(m[i], m[32 + i]), fmaxf(m[64 + i], m[96 + i]));
+    };
+    if (on) {
+      const float magic = row_magic(row_bound());
+      float dummy = 0.f;
+#pragma unroll
+      for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 8 * c, magic, dummy);
+    }
+    bool tr_pending = false;
+    auto trace_check = [&]() {
+      if (t == 0 && fabs(S.trp[0] + S.trp[1] - S.tr0) > a.trace_tol * fmax(1.0, fabs(S.tr0)))
+        flags |= LIME_FLAG_TRACE_DRIFT;
+      tr_pending = false;
+    };
+
+#pragma unroll 1
+    for (int step = 0; step < a.n_steps; ++step) {
+#pragma unroll 1
+      for (int s = 0; s < 4; ++s, ++g) {
+        tc::fence_proxy_async_smem();
+        tc::tc_fence_before();
+        __syncthreads();
+        if (t == 0) {
+          tc::tc_fence_after();
+          small_mma<kW, kDual>(tbase, desc_b0, desc_b1, true, kDual);
+          tc::mma_commit(&S.mbar);
+        }
+        if (tr_pending) trace_check();
+        const float magic = row_magic(row_bound());
+        int timed_out = tc::mbar_wait_bounded(&S.mbar, phase, a.max_wait) ? 0 : 1;
+        phase ^= 1u;
+        tc::tc_fence_after();
+        float v1[kC], v[kC];
+        if (kDual) {
+          uint32_t r0[kC / 8][8], r1[kC / 8][8];
+#pragma unroll
+          for (int c = 0; c < kC / 8; ++c) {
+            tc::tmem_ld8_nowait(lane_addr + Sh::kD1 + j0 + 8 * c, r1[c]);
+            tc::tmem_ld8_nowait(lane_addr + Sh::kD + j0 + 8 * c, r0[c]);
+          }
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int c = 0; c < kC; ++c) {
+            v1[c] = __uint_as_float(r1[c / 8][c % 8]);
+            v[c] = __uint_as_float(r0[c / 8][c % 8]);
+          }
+        } else {
+          tmem_ld<kC>(lane_addr + Sh::kD1 + j0, v1);
+          tc::tc_fence_before();
+          if (__syncthreads_or(timed_out)) {
+            aborted = true;
+            break;
+          }
+          if (t == 0) {
+            tc::tc_fence_after();
+            small_mma<kW, kDual>(tbase, desc_b0, desc_b1, false, true);
+            tc::mma_commit(&S.mbar);
+          }
+          timed_out = tc::mbar_wait_bounded(&S.mbar, phase, a.max_wait) ? 0 : 1;
+          phase ^= 1u;
+          tc::tc_fence_after();
+          tmem_ld<kC>(lane_addr + Sh::kD + j0, v);
+        }
+        float own[kC];
+#pragma unroll
+        for (int c = 0; c < kC; ++c) own[c] = __fadd_rn(v[c], v1[c]);
+        // dephasing jump term, folded into the diagonal of X (in column j0 + jj = i)
+        if (diag_owner)
+#pragma unroll
+          for (int jj = 0; jj < kC; ++jj)
+            if (j0 + jj == i) own[jj] = __fmaf_rn(mi * a.sa_half, rs_d, own[jj]);
+        if (on)
+#pragma unroll
+          for (int e = 0; e < kC / 4; ++e)
+            *reinterpret_cast<float4*>(xrow + j0 + 4 * e) =
+                make_float4(own[4 * e], own[4 * e + 1], own[4 * e + 2], own[4 * e + 3]);
+        if (__syncthreads_or(timed_out)) {
+          aborted = true;
+          break;
+        }
+        float nmx = 0.f;
+        if (on) {
+          float u[kC];
+#pragma unroll
+          for (int jj = 0; jj < kC; ++jj) u[jj] = __fmaf_rn(tsign, xcol[(j0 + jj) * kLd], own[jj]);
+          if (s < 3) {
+            const float cst = (s == 2) ? a.c_full : a.c_half;
+            const float wgt = (s == 0) ? 1.f : 2.f;
+            if (diag_owner) {
+              const float xd = xrow[i];
+              const float ud = __fadd_rn(xd, xd);
+              acc_d = __fmaf_rn(wgt, ud, acc_d);
+              rs_d = __fmaf_rn(cst, ud, rho_d);
+            }
+#pragma unroll
+            for (int jj = 0; jj < kC; ++jj) {
+              acc[jj] = __fmaf_rn(wgt, u[jj], acc[jj]);
+              u[jj] = __fmaf_rn(cst, u[jj], rho[jj]);
+            }
+#pragma unroll
+            for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, u + 8 * c, magic, nmx);
+          } else {
+            if (diag_owner) {
+              const float xd = xrow[i];
+              float lo_d = S.rlo[(i - j0) * 128 + t];
+              rho_d = rk4_final_f32(rho_d, acc_d, __fadd_rn(xd, xd), a.c_sixth, a.c_sixth_lo, lo_d);
+              acc_d = 0.f;
+              rs_d = rho_d;
+            }
+#pragma unroll
+            for (int jj = 0; jj < kC; ++jj) {
+              float lo = S.rlo[jj * 128 + t];
+              rho[jj] = rk4_final_f32(rho[jj], acc[jj], u[jj], a.c_sixth, a.c_sixth_lo, lo);
+              S.rlo[jj * 128 + t] = lo;
+              acc[jj] = 0.f;
+            }
+#pragma unroll
+            for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 8 * c, magic, nmx);
+          }
+        }
+        S.smax[(g + 1) & 1][t] = nmx;
+      }
+      if (aborted) break;
+
+      // ---- observables / trace after the step ----
+      const int gstep = a.step0 + step;
+      if (((gstep + 1) % a.obs_every) == 0) {
+        const int slot = (gstep + 1) / a.obs_every - 1;
+        double2* orow = a.obs_out + ((int64_t)b * a.obs_per_inst + slot) * a.n_obs;
+        const size_t obase = ((size_t)b * a.obs_per_inst + slot) * a.n_obs;
+        const double dval =
+            diag_owner ? fpconv::scale_pow2(fpconv::widen_f32(rho_d) + fpconv::widen_f32(S.rlo[(i - j0) * 128 + t]),
+                                            -S.eb)
+                       : 0.0;
+        if (a.obs_mode == 1) {
+          if (diag_owner && i < a.n_obs && in_bounds((obase + i) * 16, 16, a.obs_elems * 16, a.status))
+            orow[i] = make_double2(dval, 0.0);
+        } else if (a.obs_mode == 2) {
+          const double2* E0 = a.obs_ops + p * a.obs_stride;
+          for (int o = 0; o < a.n_obs; ++o) {
+            const double2* E = E0 + (int64_t)o * n * n;
+            float pr = 0.f, pi = 0.f;
+            // the row's sum in column order: the first half, then on from its value
+#pragma unroll 1
+            for (int part = 0; part < 2; ++part) {
+              if (part == h && i < n) {
+                if (h) {
+                  pr = S.obsp[0][t - 32];
+                  pi = S.obsp[1][t - 32];
+                }
+#pragma unroll
+                for (int jj = 0; jj < kC; ++jj) {
+                  const int j = j0 + jj;
+                  if (j < n) {
+                    const double2 ev = E[(int64_t)j * n + i];   // E[j][i]
+                    const float er = (float)ev.x, ei = (float)ev.y;
+                    if (is_re) {
+                      pr = __fmaf_rn(er, rho[jj], pr);
+                      pi = __fmaf_rn(ei, rho[jj], pi);
+                    } else {
+                      pr = __fmaf_rn(ei, rho[jj], pr);
+                      pi = __fmaf_rn(-er, rho[jj], pi);
+                    }
+                  }
+                }
+                if (!h) {
+                  S.obsp[0][t] = pr;
+                  S.obsp[1][t] = pi;
+                  pr = pi = 0.f;
+                }
+              }
+              if (part == 0) __syncthreads();
+            }
+            const double sr = fpconv::scale_pow2(block_sum<4>((double)pr, S.red[0], t), -S.eb);
+            const double si = fpconv::scale_pow2(block_sum<4>((double)pi, S.red[1], t), -S.eb);
+            if (t == 0 && in_bounds((obase + o) * 16, 16, a.obs_elems * 16, a.status)) orow[o] = make_double2(sr, si);
+          }
+        }
+        if (a.trace_tol > 0.0) {
+          if (is_re) {
+            double v = (diag_owner && i < n) ? dval : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (i == 0) S.trp[h] = v;
+          }
+          tr_pending = true;
+        }
+      }
+    }
+    if (aborted) break;
+
+    // ---- final state ----
+    __syncthreads();   // the last stage's reads of the transpose buffer are done
+    if (on) {
+      double* sd = reinterpret_cast<double*>(stg);
+      const int comp = is_re ? 0 : 1;
+      const int ebi = -S.eb;
+      const uint64_t neg = is_re ? 0ull : 0x8000000000000000ull;
+#pragma unroll
+      for (int jj = 0; jj < kC; ++jj) {
+        const double v = fpconv::scale_pow2(fpconv::widen_f32(rho[jj]) + fpconv::widen_f32(S.rlo[jj * 128 + t]), ebi);
+        if (!isfinite(rho[jj])) flags |= LIME_FLAG_NONFINITE;
+        sd[2 * at(i, j0 + jj) + comp] = fpconv::from_bits64(fpconv::bits64(v) ^ neg);
+      }
+    }
+    __syncthreads();
+    {
+      double2* out = a.rho_out + (int64_t)b * n * n;
+      for (int e = t; e < n * n; e += Sh::kThreads) {
+        const int ii = e / n, jj = e - ii * n;
+        if (in_bounds(((size_t)b * n * n + e) * 16, 16, a.rho_elems * 16, a.status)) out[e] = stg[at(ii, jj)];
+      }
+    }
+    __syncthreads();   // smax / rlo of this instance are no longer read
+    if (tr_pending) trace_check();
+  }
+
+  if (aborted) {
+    flags |= LIME_FLAG_TIMEOUT;
+    if (t == 0) tc::mbar_wait_bounded(&S.mbar, phase ^ 1u, a.max_wait);
+  }
+  if (flags) atomicOr(a.status, flags);
+  tc::tc_fence_before();
+  __syncthreads();
+  if (q == 0) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tbase, Sh::kTmem);
+  }
+}
+
 // ---------------------------------------------------------------- drive preparation
 // Workspace of a driven call: fp32 hi/lo pairs of Heff ([P|1][2][64][64]),
 // of the drive operators ([n_drive][2][64][64]) and of the coefficients
@@ -1079,10 +1558,27 @@ extern "C" int lime_lindblad_rk4_split(const LimeLindbladSplitDesc* d, void* str
     LIME_CUDA_TRY(cudaGetLastError());
     count_launch(5);
   }
-  const int ctas_per_sm = d->ctas_per_sm > 0 ? d->ctas_per_sm : 2;
+  // Dimensions up to 32 without a drive leave the 64-wide kernel, whose time
+  // does not depend on n (20 steps of 16 instances 0.35 ms, of 4096 4.7 ms; at
+  // n = 16 0.17 and 0.72, at n = 32 0.21 and 1.40 ms).  One wait a stage
+  // (kDual) while its CTAs hold the batch in one round; beyond that the other
+  // form holds twice as many (n = 32, 608 instances in one round: 0.27 ms,
+  // where 304 in one round of the first take 0.22).
+  void (*kern)(split::Args) = driven ? split::lindblad_rk4_split_kernel<true> : split::lindblad_rk4_split_kernel<false>;
+  size_t smem = sizeof(split::Smem) + 1024;
+  int threads = split::kThreads, resident = 2;
+  if (!driven && d->n <= 32) {
+    const bool w16 = d->n <= 16;
+    const bool dual = d->batch <= (w16 ? split::SmallShape<16, true>::kCtas : split::SmallShape<32, true>::kCtas) * g_num_sms;
+    kern = w16 ? (dual ? split::lindblad_rk4_split_small_kernel<16, true> : split::lindblad_rk4_split_small_kernel<16, false>)
+               : (dual ? split::lindblad_rk4_split_small_kernel<32, true> : split::lindblad_rk4_split_small_kernel<32, false>);
+    smem = (w16 ? sizeof(split::SmallSmem<16>) : sizeof(split::SmallSmem<32>)) + 128;
+    threads = 128;
+    resident = w16 ? (dual ? split::SmallShape<16, true>::kCtas : split::SmallShape<16, false>::kCtas)
+                   : (dual ? split::SmallShape<32, true>::kCtas : split::SmallShape<32, false>::kCtas);
+  }
+  const int ctas_per_sm = d->ctas_per_sm > 0 ? d->ctas_per_sm : resident;
   const int grid = (int)((d->batch < ctas_per_sm * g_num_sms) ? d->batch : ctas_per_sm * g_num_sms);
-  const size_t smem = sizeof(split::Smem) + 1024;
-  auto kern = driven ? split::lindblad_rk4_split_kernel<true> : split::lindblad_rk4_split_kernel<false>;
   LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // bounded launches: about 2^22 instance-steps per launch
   const double per_cta = (double)((d->batch + grid - 1) / grid);
@@ -1092,7 +1588,7 @@ extern "C" int lime_lindblad_rk4_split(const LimeLindbladSplitDesc* d, void* str
   for (int s0 = 0; s0 < d->n_steps; s0 += chunk) {
     a.step0 = s0;
     a.n_steps = (d->n_steps - s0 < chunk) ? d->n_steps - s0 : chunk;
-    kern<<<grid, split::kThreads, smem, st>>>(a);
+    kern<<<grid, threads, smem, st>>>(a);
     LIME_CUDA_TRY(cudaGetLastError());
     count_launch();
     a.rho = a.rho_out;   // the next launch continues from this one's final state
