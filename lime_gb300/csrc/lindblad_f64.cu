@@ -1,11 +1,12 @@
-// FP64 Lindblad adjoint (one CTA per density matrix: CTA-wide complex GEMMs,
-// register-tiled, operands staged through shared memory) and the preparation
-// of the generators.
+// FP64 Lindblad adjoint with dense collapse operators (one CTA per density
+// matrix: CTA-wide complex GEMMs, register-tiled, operands staged through
+// shared memory; without them see lindblad_adjoint_rows_f64.cu) and the
+// preparation of the generators.
 //
 // GB300 executes FP64 at a small fraction of its tensor rate, so this path is
 // DFMA-bound; its job is to be exact.
 
-#include "common.cuh"
+#include "adjoint_f64.cuh"
 
 namespace lime {
 namespace f64 {
@@ -110,29 +111,6 @@ __device__ void apply_gen(const Gen& G, const double2* x, double2* out, double2*
     out[e] = f;
   }
   __syncthreads();
-}
-
-struct AdjArgs {
-  int n, param_batch, seg_steps, step0, total_steps, k_dense, n_obs, obs_diag, obs_every, obs_per_inst;
-  double dt;
-  const double2* ckpt;
-  double2* lam;
-  const double2* heff; int64_t heff_stride;
-  const double2* m; int64_t m_stride;
-  const double2* ld; int64_t ld_stride;
-  const double2* heff_adj; int64_t heff_adj_stride;
-  const double2* m_adj; int64_t m_adj_stride;
-  const double2* ld_adj; int64_t ld_adj_stride;
-  const double2* obs_ops; int64_t obs_stride;
-  const double2* obs_grad;
-  double* g_diag;
-  double* g_bond;
-  double* g_gamma;
-  double2* ws;
-};
-
-__host__ __device__ inline int64_t adj_ws_mats(int seg_steps, int k_dense) {
-  return (int64_t)seg_steps + 9 + (k_dense > 0 ? 2 : 0);
 }
 
 // Parameter-gradient contributions of one stage: abar = adjoint of the stage
@@ -433,6 +411,9 @@ extern "C" int lime_lindblad_adjoint_f64(const LimeAdjointDesc* d, void* stream)
   a.g_diag = d->grad_diag; a.g_bond = d->grad_bond; a.g_gamma = d->grad_gamma;
   a.ws = reinterpret_cast<double2*>(d->workspace);
   cudaStream_t st = (cudaStream_t)stream;
+  // Without dense operators the products run over the generators' nonzero
+  // entries; a dense Heff costs half the tiles' FP64 work there too.
+  if (d->k_dense == 0) return f64::launch_adjoint_rows(a, d->batch, st);
   if (d->n <= 16) return launch_adj<1>(a, d->batch, st);
   if (d->n <= 32) return launch_adj<2>(a, d->batch, st);
   return launch_adj<4>(a, d->batch, st);
