@@ -14,9 +14,8 @@
 //   warp 0      producer: bulk copies of 5 pieces per K chunk (80 KB)
 //   warp 1      MMA issuer: tcgen05.mma M=128 N=128 K=16, kind::f16
 //   warps 2..17 epilogue: drain TMEM accumulators into fp32 two-sum
-//               accumulators (hi words in registers, lo words in shared
-//               memory), then park the finished tile in shared memory for
-//               the caller's fused epilogue.
+//               accumulators in registers, then park the finished tile in
+//               shared memory for the caller's fused epilogue.
 //
 // Precision.  A = A0 (per-row 7-bit fixed point, 64 k with |k| <= 127 after
 // the row's power-of-two scaling) + A1 + A2 (fp16 residuals); B = B0
@@ -31,6 +30,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "fpconv.cuh"
 #include "tc_ptx.cuh"
 
@@ -75,7 +75,7 @@ static_assert(kCK % 16 == 0 && 128 % kCK == 0, "K chunks are whole MMA K steps a
 
 struct __align__(1024) Smem {
   uint8_t stage[kStages][5][kPiece];               // A0 A1 A2 B0 B1; the parked tile after the last MMA
-  float lo[kBN * kBM];                             // low words of the fp32 two-sum accumulators, [col][row]
+  float lo[kBN * kBM];                             // parked tile of a sequence, or its low words (park_split), [col][row]
   uint64_t full[kStages], empty[kStages], accf[2], acce[2], drain;
   uint32_t tmem_base;
   int abort;
@@ -193,6 +193,17 @@ __device__ __forceinline__ void rk4_stage8(const RK4& k, float* Phi, float* Plo,
   }
 }
 
+// Descriptor of K step ks of piece i of the ring stage at `base` (its low
+// word): one addition an operand, so that the issuing thread, which competes
+// with the epilogue warps, keeps up with the tensor core.
+__device__ __forceinline__ uint32_t operand_base(const void* stage) {
+  return (tc::smem_u32(stage) & 0x3FFFFu) >> 4 | (kLBO >> 4) << 16;
+}
+__device__ __forceinline__ uint64_t operand(uint32_t base, int i, int ks) {
+  constexpr uint64_t hi = (uint64_t)((kSBO >> 4) | (1u << 14)) << 32;
+  return hi | (base + (uint32_t)((i * kPiece + ks * 2 * kLBO) >> 4));
+}
+
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
 
 // The operands and scaling of one tile.
@@ -213,6 +224,40 @@ struct Tile {
   // that combine tiles with cancellation
   int park_split = 0;
 };
+
+// One 128-K accumulator group of an epilogue thread's kEpiCols columns: the
+// exact D0 (at d0) enters the fp32 two-sum, D1 (128 columns further) is added
+// to its low words.  The main loop's bound after the MMAs themselves (865 of
+// 1175 us of the 9216-dimensional Redfield stage run alone) is the issue
+// slots of these additions, so they are packed two to an instruction and
+// both words stay in registers: 1175 -> 961 us.  (Copies are not the bound:
+// leaving them out, or halving the L2 reads by cluster multicast, changes
+// nothing.)
+__device__ __forceinline__ void drain_group(uint32_t d0, float (&hi)[kEpiCols], float (&lo)[kEpiCols]) {
+#pragma unroll
+  for (int q = 0; q < kEpiCols / 8; ++q) {
+    uint32_t v[8];
+    uint64_t er[4];
+    tc::tmem_ld8_nowait(d0 + 8 * q, v);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = 8 * q + 2 * e;
+      const uint64_t h = x2::pack(hi[c], hi[c + 1]), x = (uint64_t)v[2 * e + 1] << 32 | v[2 * e];
+      const uint64_t sm = x2::add(h, x), bv = x2::sub(sm, h);
+      er[e] = x2::add(x2::sub(h, x2::sub(sm, bv)), x2::sub(x, bv));
+      x2::unpack(sm, hi[c], hi[c + 1]);
+    }
+    tc::tmem_ld8_nowait(d0 + 128u + 8 * q, v);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = 8 * q + 2 * e;
+      const uint64_t d1 = (uint64_t)v[2 * e + 1] << 32 | v[2 * e];
+      x2::unpack(x2::add(x2::pack(lo[c], lo[c + 1]), x2::add(er[e], d1)), lo[c], lo[c + 1]);
+    }
+  }
+}
 
 // TMEM allocation and barrier set-up; every thread of the CTA calls it.
 __device__ __forceinline__ void setup(Smem& S) {
@@ -308,21 +353,15 @@ __device__ __forceinline__ bool mainloop(Smem& S, const Tile& T) {
         tc::tc_fence_after();
         const uint32_t d0 = tbase + (uint32_t)(2 * b) * 128u;
         const uint32_t d1 = d0 + 128u;
-        const uint32_t base = tc::smem_u32(S.stage[s][0]);
+        const uint32_t base = operand_base(S.stage[s][0]);
 #pragma unroll
         for (int ks = 0; ks < kCK / 16; ++ks) {
-          const uint32_t ko = (uint32_t)ks * 2u * kLBO;
-          const uint64_t a0 = tc::smem_desc_noswizzle(base + 0 * kPiece + ko, kLBO, kSBO);
-          const uint64_t a1 = tc::smem_desc_noswizzle(base + 1 * kPiece + ko, kLBO, kSBO);
-          const uint64_t a2 = tc::smem_desc_noswizzle(base + 2 * kPiece + ko, kLBO, kSBO);
-          const uint64_t b0 = tc::smem_desc_noswizzle(base + 3 * kPiece + ko, kLBO, kSBO);
-          const uint64_t b1 = tc::smem_desc_noswizzle(base + 4 * kPiece + ko, kLBO, kSBO);
           const uint32_t acc = (first && ks == 0) ? 0u : 1u;
-          tc::mma_f16_ss(d0, a0, b0, idesc, acc);
-          tc::mma_f16_ss(d1, a1, b0, idesc, acc);
-          tc::mma_f16_ss(d1, a0, b1, idesc, 1u);
-          tc::mma_f16_ss(d1, a1, b1, idesc, 1u);
-          tc::mma_f16_ss(d1, a2, b0, idesc, 1u);
+          tc::mma_f16_ss(d0, operand(base, 0, ks), operand(base, 3, ks), idesc, acc);
+          tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 3, ks), idesc, acc);
+          tc::mma_f16_ss(d1, operand(base, 0, ks), operand(base, 4, ks), idesc, 1u);
+          tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 4, ks), idesc, 1u);
+          tc::mma_f16_ss(d1, operand(base, 2, ks), operand(base, 3, ks), idesc, 1u);
         }
         tc::mma_commit(&S.empty[s]);
         if (last) tc::mma_commit(&S.accf[b]);
@@ -339,12 +378,9 @@ __device__ __forceinline__ bool mainloop(Smem& S, const Tile& T) {
   const int h = (warp - 2) >> 2;                  // column group of kEpiCols
   const int r = lq * 32 + lane;
   const uint32_t lane_addr = tbase + ((uint32_t)(lq * 32) << 16);
-  // hi words in registers, lo words in shared memory (each thread owns its
-  // 64 entries; lanes hit consecutive words)
-  float hi[kEpiCols];
-  float* lo = S.lo + (kEpiCols * h) * kBM + r;
+  float hi[kEpiCols], lo[kEpiCols];
 #pragma unroll
-  for (int c = 0; c < kEpiCols; ++c) { hi[c] = 0.f; lo[c * kBM] = 0.f; }
+  for (int c = 0; c < kEpiCols; ++c) hi[c] = lo[c] = 0.f;
   const int n_groups = KC / kGroup;
   bool ok = true;
   for (int p = 0; p < n_groups; ++p) {
@@ -355,29 +391,7 @@ __device__ __forceinline__ bool mainloop(Smem& S, const Tile& T) {
       break;
     }
     tc::tc_fence_after();
-    const uint32_t d0 = lane_addr + (uint32_t)(2 * b) * 128u + (uint32_t)(kEpiCols * h);
-#pragma unroll
-    for (int q = 0; q < kEpiCols / 16; ++q) {
-      // (one load and wait per accumulator measured faster than both loads
-      // under one wait)
-      float v[16], er[16];
-      tc::tmem_ld16(d0 + 16 * q, v);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        // exact D0 into the two-sum
-        const float x = v[e];
-        const float sm = __fadd_rn(hi[16 * q + e], x);
-        const float bv = __fsub_rn(sm, hi[16 * q + e]);
-        er[e] = __fadd_rn(__fsub_rn(hi[16 * q + e], __fsub_rn(sm, bv)), __fsub_rn(x, bv));
-        hi[16 * q + e] = sm;
-      }
-      tc::tmem_ld16(d0 + 128u + 16 * q, v);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        float* l = lo + (16 * q + e) * kBM;
-        *l = __fadd_rn(*l, __fadd_rn(er[e], v[e]));
-      }
-    }
+    drain_group(lane_addr + (uint32_t)(2 * b) * 128u + (uint32_t)(kEpiCols * h), hi, lo);
     tc::tc_fence_before();
     tc::mbar_arrive(&S.acce[b]);
   }
@@ -390,12 +404,12 @@ __device__ __forceinline__ bool mainloop(Smem& S, const Tile& T) {
 #pragma unroll
       for (int c = 0; c < kEpiCols; ++c) {
         ft[(kEpiCols * h + c) * kFStride + r] = __fmul_rn(hi[c], rs);
-        lo[c * kBM] = __fmul_rn(lo[c * kBM], rs);
+        S.lo[(kEpiCols * h + c) * kBM + r] = __fmul_rn(lo[c], rs);
       }
     } else {
 #pragma unroll
       for (int c = 0; c < kEpiCols; ++c)
-        ft[(kEpiCols * h + c) * kFStride + r] = __fmul_rn(__fadd_rn(hi[c], lo[c * kBM]), rs);
+        ft[(kEpiCols * h + c) * kFStride + r] = __fmul_rn(__fadd_rn(hi[c], lo[c]), rs);
     }
   }
   epi_bar();
@@ -502,21 +516,15 @@ __device__ __forceinline__ bool seq_mma(Smem& S, const Tile& T, Seq& q) {
     tc::tc_fence_after();
     const uint32_t d0 = tbase + (uint32_t)(2 * b) * 128u;
     const uint32_t d1 = d0 + 128u;
-    const uint32_t base = tc::smem_u32(S.stage[s][0]);
+    const uint32_t base = operand_base(S.stage[s][0]);
 #pragma unroll
     for (int ks = 0; ks < kCK / 16; ++ks) {
-      const uint32_t ko = (uint32_t)ks * 2u * kLBO;
-      const uint64_t a0 = tc::smem_desc_noswizzle(base + 0 * kPiece + ko, kLBO, kSBO);
-      const uint64_t a1 = tc::smem_desc_noswizzle(base + 1 * kPiece + ko, kLBO, kSBO);
-      const uint64_t a2 = tc::smem_desc_noswizzle(base + 2 * kPiece + ko, kLBO, kSBO);
-      const uint64_t b0 = tc::smem_desc_noswizzle(base + 3 * kPiece + ko, kLBO, kSBO);
-      const uint64_t b1 = tc::smem_desc_noswizzle(base + 4 * kPiece + ko, kLBO, kSBO);
       const uint32_t acc = (first && ks == 0) ? 0u : 1u;
-      tc::mma_f16_ss(d0, a0, b0, idesc, acc);
-      tc::mma_f16_ss(d1, a1, b0, idesc, acc);
-      tc::mma_f16_ss(d1, a0, b1, idesc, 1u);
-      tc::mma_f16_ss(d1, a1, b1, idesc, 1u);
-      tc::mma_f16_ss(d1, a2, b0, idesc, 1u);
+      tc::mma_f16_ss(d0, operand(base, 0, ks), operand(base, 3, ks), idesc, acc);
+      tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 3, ks), idesc, acc);
+      tc::mma_f16_ss(d1, operand(base, 0, ks), operand(base, 4, ks), idesc, 1u);
+      tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 4, ks), idesc, 1u);
+      tc::mma_f16_ss(d1, operand(base, 2, ks), operand(base, 3, ks), idesc, 1u);
     }
     tc::mma_commit(&S.empty[s]);
     if (last) {
@@ -544,12 +552,9 @@ __device__ __forceinline__ bool seq_drain(Smem& S, const Tile& T, Seq& q) {
   const int h = (warp - 2) >> 2;
   const int r = lq * 32 + lane;
   const uint32_t lane_addr = S.tmem_base + ((uint32_t)(lq * 32) << 16);
-  float hi[kEpiCols];
+  float hi[kEpiCols], lo[kEpiCols];
 #pragma unroll
-  for (int c = 0; c < kEpiCols; ++c) {
-    hi[c] = 0.f;
-    S.lo[park_idx(kEpiCols * h + c, r)] = 0.f;
-  }
+  for (int c = 0; c < kEpiCols; ++c) hi[c] = lo[c] = 0.f;
   const int n_groups = T.n_chunks / kGroup;
   bool ok = true;
   for (int p = 0; p < n_groups; ++p, ++q.gp) {
@@ -560,26 +565,7 @@ __device__ __forceinline__ bool seq_drain(Smem& S, const Tile& T, Seq& q) {
       break;
     }
     tc::tc_fence_after();
-    const uint32_t d0 = lane_addr + (uint32_t)(2 * b) * 128u + (uint32_t)(kEpiCols * h);
-#pragma unroll
-    for (int qq = 0; qq < kEpiCols / 16; ++qq) {
-      float v[16], er[16];
-      tc::tmem_ld16(d0 + 16 * qq, v);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const float x = v[e];
-        const float sm = __fadd_rn(hi[16 * qq + e], x);
-        const float bv = __fsub_rn(sm, hi[16 * qq + e]);
-        er[e] = __fadd_rn(__fsub_rn(hi[16 * qq + e], __fsub_rn(sm, bv)), __fsub_rn(x, bv));
-        hi[16 * qq + e] = sm;
-      }
-      tc::tmem_ld16(d0 + 128u + 16 * qq, v);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        float* l = S.lo + park_idx(kEpiCols * h + 16 * qq + e, r);
-        *l = __fadd_rn(*l, __fadd_rn(er[e], v[e]));
-      }
-    }
+    drain_group(lane_addr + (uint32_t)(2 * b) * 128u + (uint32_t)(kEpiCols * h), hi, lo);
     tc::tc_fence_before();
     tc::mbar_arrive(&S.acce[b]);
   }
@@ -587,8 +573,7 @@ __device__ __forceinline__ bool seq_drain(Smem& S, const Tile& T, Seq& q) {
     const float rs = __fmul_rn(T.row_inv[r], T.inv_sb);
 #pragma unroll
     for (int c = 0; c < kEpiCols; ++c) {
-      float* l = S.lo + park_idx(kEpiCols * h + c, r);
-      *l = __fmul_rn(__fadd_rn(hi[c], *l), rs);
+      S.lo[park_idx(kEpiCols * h + c, r)] = __fmul_rn(__fadd_rn(hi[c], lo[c]), rs);
     }
   }
   epi_bar();
