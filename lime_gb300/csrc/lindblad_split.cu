@@ -53,8 +53,13 @@
 // accumulator units (X = 2^(a+b) Heff rho): the conversion factors are powers
 // of two folded into dt/2, dt and dt/6, so the epilogue multiplies by no scale
 // and the results are those of the natural-unit arithmetic scaled exactly.
+//
+// The epilogue's issue slots are the second bound beside the latency of a
+// stage, so its arithmetic runs on pairs of columns (f32x2.cuh): 4096
+// instances of 64 levels, 20 steps, 4.77 -> 4.48 ms.
 
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "fpconv.cuh"
 #include "tc_ptx.cuh"
 
@@ -171,21 +176,45 @@ __device__ __forceinline__ float row_magic(float m) {
   return ldexpf(1.5f, e + 14);
 }
 
-// Split 8 consecutive B^T values into b0 (q grid) + b1 (fp16 residual) and store.
+// Split 8 consecutive B^T values (pairs) into b0 (q grid) + b1 (fp16 residual) and store.
 template <class SmemT>
-__device__ __forceinline__ void store_b8(SmemT& S, uint32_t off, const float* x, float magic, float& mx) {
+__device__ __forceinline__ void store_b8(SmemT& S, uint32_t off, const uint64_t* x, float magic, float& mx) {
+  const uint64_t up = x2::both(magic), down = x2::both(-magic);
   uint32_t h0[4], h1[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const float u = x[2 * e], w = x[2 * e + 1];
-    const float u0 = __fsub_rn(__fadd_rn(u, magic), magic);
-    const float w0 = __fsub_rn(__fadd_rn(w, magic), magic);
+    const uint64_t g = x2::add(x2::add(x[e], up), down), d = x2::sub(x[e], g);
+    float u, w, u0, w0, u1, w1;
+    x2::unpack(x[e], u, w);
+    x2::unpack(g, u0, w0);
+    x2::unpack(d, u1, w1);
     h0[e] = pack_f2h2(u0, w0);
-    h1[e] = pack_f2h2(__fsub_rn(u, u0), __fsub_rn(w, w0));
+    h1[e] = pack_f2h2(u1, w1);
     mx = fmaxf(mx, fmaxf(fabsf(u), fabsf(w)));
   }
   *reinterpret_cast<uint4*>(S.bop[0] + off) = make_uint4(h0[0], h0[1], h0[2], h0[3]);
   *reinterpret_cast<uint4*>(S.bop[1] + off) = make_uint4(h1[0], h1[1], h1[2], h1[3]);
+}
+
+// value jj of a row held as pairs
+__device__ __forceinline__ float at(const uint64_t* v, int jj) {
+  float a, b;
+  x2::unpack(v[jj >> 1], a, b);
+  return jj & 1 ? b : a;
+}
+
+// rk4_final_f32 on two elements
+__device__ __forceinline__ uint64_t rk4_final_f32x2(uint64_t x, uint64_t acc, uint64_t f, uint64_t c6, uint64_t c6lo,
+                                                    uint64_t& lo) {
+  const uint64_t ksum = x2::add(acc, f), inc = x2::mul(ksum, c6);
+  const uint64_t inc_res = x2::fma(ksum, c6, x2::mul(inc, x2::both(-1.f)));
+  const uint64_t inc_lo = x2::fma(ksum, c6lo, inc_res);
+  const uint64_t sum = x2::add(x, inc), bv = x2::sub(sum, x);
+  const uint64_t err = x2::add(x2::sub(x, x2::sub(sum, bv)), x2::sub(inc, bv));
+  const uint64_t l = x2::add(lo, x2::add(err, inc_lo));
+  const uint64_t hi2 = x2::add(sum, l);
+  lo = x2::sub(l, x2::sub(hi2, sum));
+  return hi2;
 }
 
 // x -= c * m on double-float pairs (x = xh + xl, c = ch + cl, m = mh + ml;
@@ -524,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
       }
     }
     __syncthreads();
-    float rho[kCols], acc[kCols];
+    uint64_t rho[kCols / 2], acc[kCols / 2];   // pairs of columns
     double dtr = 0.0;
     float fro = 0.f;
     bool herm = true;   // rho_ji = conj rho_ij, compared bit for bit (+0 == -0)
@@ -533,19 +562,23 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
       const int comp = is_re ? 0 : 1;
       const uint64_t flip = is_re ? 0ull : 0x8000000000000000ull;
 #pragma unroll
-      for (int jj = 0; jj < kCols; ++jj) {
-        const int j = j0 + jj;
-        const double v = sd[2 * stage_index(i, j) + comp];
-        const uint64_t bv = fpconv::bits64(v);
-        const uint64_t bw = fpconv::bits64(sd[2 * stage_index(j, i) + comp]) ^ flip;
-        herm &= (bv == bw) || ((bv | bw) << 1) == 0;
-        float hv, lv;
-        fpconv::split_f64(v, hv, lv);   // (float) v and (float)(v - hv) without FP64 instructions
-        rho[jj] = hv;
-        acc[jj] = 0.f;
-        S.rlo[j * 128 + r] = lv;
-        fro = __fmaf_rn(hv, hv, fro);
-        if (diag_owner && j == i) dtr = v;
+      for (int k = 0; k < kCols / 2; ++k) {
+        float hv[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int j = j0 + 2 * k + q;
+          const double v = sd[2 * stage_index(i, j) + comp];
+          const uint64_t bv = fpconv::bits64(v);
+          const uint64_t bw = fpconv::bits64(sd[2 * stage_index(j, i) + comp]) ^ flip;
+          herm &= (bv == bw) || ((bv | bw) << 1) == 0;
+          float lv;
+          fpconv::split_f64(v, hv[q], lv);   // (float) v and (float)(v - hv) without FP64 instructions
+          S.rlo[j * 128 + r] = lv;
+          fro = __fmaf_rn(hv[q], hv[q], fro);
+          if (diag_owner && j == i) dtr = v;
+        }
+        rho[k] = x2::pack(hv[0], hv[1]);
+        acc[k] = 0;
       }
     }
 #pragma unroll
@@ -577,12 +610,13 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
     float mx = 0.f;
     float rho_d = 0.f, acc_d = 0.f, rs_d = 0.f;   // diagonal element (diag_owner only)
 #pragma unroll
+    for (int k = 0; k < kCols / 2; ++k) rho[k] = x2::mul(rho[k], x2::both(bsign));
+#pragma unroll
     for (int jj = 0; jj < kCols; ++jj) {
       const int j = j0 + jj;
-      rho[jj] *= bsign;
       S.rlo[j * 128 + r] *= bsign;
-      mx = fmaxf(mx, fabsf(rho[jj]));
-      if (diag_owner && j == i) rho_d = rho[jj];
+      mx = fmaxf(mx, fabsf(at(rho, jj)));
+      if (diag_owner && j == i) rho_d = at(rho, jj);
     }
     if (!herm) flags |= LIME_FLAG_NOT_HERMITIAN;
     rs_d = rho_d;
@@ -598,12 +632,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
       const float magic = row_magic(m4);
       float dummy = 0.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float x[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = rho[8 * c + e];
-        store_b8(S, brow + (bchunk0 + c) * kLBO, x, magic, dummy);
-      }
+      for (int c = 0; c < 4; ++c) store_b8(S, brow + (bchunk0 + c) * kLBO, rho + 4 * c, magic, dummy);
     }
     bool tr_pending = false;   // a trace recorded after the last step awaits its check
 
@@ -687,9 +716,9 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
           tc::tmem_ld32(lane_addr + kColD + j0, v);
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            *reinterpret_cast<float4*>(xrow + j0 + 4 * e) =
-                make_float4(__fadd_rn(v[4 * e], v1[4 * e]), __fadd_rn(v[4 * e + 1], v1[4 * e + 1]),
-                            __fadd_rn(v[4 * e + 2], v1[4 * e + 2]), __fadd_rn(v[4 * e + 3], v1[4 * e + 3]));
+            *reinterpret_cast<ulonglong2*>(xrow + j0 + 4 * e) =
+                make_ulonglong2(x2::add(x2::pack(v[4 * e], v[4 * e + 1]), x2::pack(v1[4 * e], v1[4 * e + 1])),
+                                x2::add(x2::pack(v[4 * e + 2], v[4 * e + 3]), x2::pack(v1[4 * e + 2], v1[4 * e + 3])));
         }
         // dephasing jump term m_i rho_ii folded into the diagonal of X (it
         // enters Re f_ii = X_ii + X_ii twice, hence the half; rs_d is in B units)
@@ -716,25 +745,25 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
             acc_d = __fmaf_rn(wgt, ud, acc_d);
             rs_d_next = __fmaf_rn(cst, ud, rho_d);
           }
+          const uint64_t ts2 = x2::both(tsign), w2 = x2::both(wgt), c2 = x2::both(cst);
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            float own[16];
+            uint64_t nxt[8];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float4 o = *reinterpret_cast<const float4*>(xrow + j0 + q * 16 + 4 * e);
-              own[4 * e] = o.x; own[4 * e + 1] = o.y; own[4 * e + 2] = o.z; own[4 * e + 3] = o.w;
-            }
-            float nxt[16];
+            for (int e = 0; e < 8; e += 2) {
+              const ulonglong2 own = *reinterpret_cast<const ulonglong2*>(xrow + j0 + q * 16 + 2 * e);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int jj = q * 16 + e;
-              const float u = __fmaf_rn(tsign, xcol[(j0 + jj) * kXtStride], own[e]);
-              acc[jj] = __fmaf_rn(wgt, u, acc[jj]);
-              nxt[e] = __fmaf_rn(cst, u, rho[jj]);
+              for (int k = 0; k < 2; ++k) {
+                const int c = q * 8 + e + k, j = j0 + 2 * c;
+                const uint64_t xt = x2::pack(xcol[j * kXtStride], xcol[(j + 1) * kXtStride]);
+                const uint64_t u = x2::fma(ts2, xt, k ? own.y : own.x);
+                acc[c] = x2::fma(w2, u, acc[c]);
+                nxt[e + k] = x2::fma(c2, u, rho[c]);
+              }
             }
 #pragma unroll
             for (int h8 = 0; h8 < 2; ++h8)
-              store_b8(S, brow + (bchunk0 + 2 * q + h8) * kLBO, nxt + 8 * h8, magic, nmx);
+              store_b8(S, brow + (bchunk0 + 2 * q + h8) * kLBO, nxt + 4 * h8, magic, nmx);
           }
           rs_d = rs_d_next;
         } else {
@@ -745,26 +774,26 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
             acc_d = 0.f;
             rs_d = rho_d;
           }
+          const uint64_t ts2 = x2::both(tsign), c6 = x2::both(a.c_sixth), c6lo = x2::both(a.c_sixth_lo);
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            float own[16];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float4 o = *reinterpret_cast<const float4*>(xrow + j0 + q * 16 + 4 * e);
-              own[4 * e] = o.x; own[4 * e + 1] = o.y; own[4 * e + 2] = o.z; own[4 * e + 3] = o.w;
-            }
+            for (int e = 0; e < 8; e += 2) {
+              const ulonglong2 own = *reinterpret_cast<const ulonglong2*>(xrow + j0 + q * 16 + 2 * e);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int jj = q * 16 + e;
-              const float u = __fmaf_rn(tsign, xcol[(j0 + jj) * kXtStride], own[e]);
-              float lo = S.rlo[(j0 + jj) * 128 + r];
-              rho[jj] = rk4_final_f32(rho[jj], acc[jj], u, a.c_sixth, a.c_sixth_lo, lo);
-              S.rlo[(j0 + jj) * 128 + r] = lo;
-              acc[jj] = 0.f;
+              for (int k = 0; k < 2; ++k) {
+                const int c = q * 8 + e + k, j = j0 + 2 * c;
+                const uint64_t xt = x2::pack(xcol[j * kXtStride], xcol[(j + 1) * kXtStride]);
+                float* const l = S.rlo + j * 128 + r;
+                uint64_t lo = x2::pack(l[0], l[128]);
+                rho[c] = rk4_final_f32x2(rho[c], acc[c], x2::fma(ts2, xt, k ? own.y : own.x), c6, c6lo, lo);
+                x2::unpack(lo, l[0], l[128]);
+                acc[c] = 0;
+              }
             }
 #pragma unroll
             for (int h8 = 0; h8 < 2; ++h8)
-              store_b8(S, brow + (bchunk0 + 2 * q + h8) * kLBO, rho + q * 16 + 8 * h8, magic, nmx);
+              store_b8(S, brow + (bchunk0 + 2 * q + h8) * kLBO, rho + q * 8 + 4 * h8, magic, nmx);
           }
         }
         S.smax[(g + 1) & 1][t] = nmx;
@@ -797,11 +826,11 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
                   const float er = (float)ev.x, ei = (float)ev.y;
                   // B units: rho[jj] = 2^b Re rho_ij, or -2^b Im rho_ij
                   if (is_re) {
-                    pr = __fmaf_rn(er, rho[jj], pr);
-                    pi = __fmaf_rn(ei, rho[jj], pi);
+                    pr = __fmaf_rn(er, at(rho, jj), pr);
+                    pi = __fmaf_rn(ei, at(rho, jj), pi);
                   } else {
-                    pr = __fmaf_rn(ei, rho[jj], pr);
-                    pi = __fmaf_rn(-er, rho[jj], pi);
+                    pr = __fmaf_rn(ei, at(rho, jj), pr);
+                    pi = __fmaf_rn(-er, at(rho, jj), pi);
                   }
                 }
               }
@@ -838,8 +867,8 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
 #pragma unroll
       for (int jj = 0; jj < kCols; ++jj) {
         const int j = j0 + jj;
-        const double v = fpconv::scale_pow2(fpconv::widen_f32(rho[jj]) + fpconv::widen_f32(S.rlo[j * 128 + r]), ebi);
-        if (!isfinite(rho[jj])) flags |= LIME_FLAG_NONFINITE;
+        const double v = fpconv::scale_pow2(fpconv::widen_f32(at(rho, jj)) + fpconv::widen_f32(S.rlo[j * 128 + r]), ebi);
+        if (!isfinite(at(rho, jj))) flags |= LIME_FLAG_NONFINITE;
         sd[2 * stage_index(i, j) + comp] = fpconv::from_bits64(fpconv::bits64(v) ^ neg);
       }
     }
@@ -888,8 +917,8 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
 //
 // Bound: a stage's chain of MMA, TMEM load, transpose and B store (one
 // instance), the issue slots of the epilogue (batches).  Measured against the
-// 64-wide kernel: 4096 instances, 20 steps, n = 16: 4.66 -> 0.72 ms, n = 32:
-// 4.70 -> 1.40 ms; one 16-site chain 3.1 -> 1.0 us a stage.
+// 64-wide kernel: 4096 instances, 20 steps, n = 16: 4.66 -> 0.69 ms, n = 32:
+// 4.70 -> 1.36 ms; one 16-site chain 3.1 -> 1.0 us a stage.
 template <int kW>
 struct __align__(128) SmallSmem {
   uint8_t bop[2][4 * kW * kW];           // B0, B1: kW (N) x 2 kW (K) fp16
@@ -983,7 +1012,7 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
   const float tsign = is_re ? 1.f : -1.f;
   float* xrow = S.xt + (on ? row : 0) * kLd;
   const float* xcol = S.xt + (is_re ? kW : 0) * kLd + (on ? i : 0);
-  auto at = [](int r, int c) { return r * kW + (c ^ (r & 7)); };   // staged element, as stage_index
+  auto pos = [](int r, int c) { return r * kW + (c ^ (r & 7)); };   // staged element, as stage_index
   uint32_t phase = 0;
   int flags = 0;
   bool aborted = false;
@@ -1040,11 +1069,11 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
         if (ii < n && jj < n &&
             in_bounds(((size_t)b * n * n + ii * n + jj) * 16, 16, a.rho_elems * 16, a.status))
           z = r0[ii * n + jj];
-        stg[at(ii, jj)] = z;
+        stg[pos(ii, jj)] = z;
       }
     }
     __syncthreads();
-    float rho[kC], acc[kC];
+    uint64_t rho[kC / 2], acc[kC / 2];
     double dtr = 0.0;
     float fro = 0.f;
     bool herm = true;
@@ -1053,25 +1082,29 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
       const int comp = is_re ? 0 : 1;
       const uint64_t flip = is_re ? 0ull : 0x8000000000000000ull;
 #pragma unroll
-      for (int jj = 0; jj < kC; ++jj) {
-        const int j = j0 + jj;
-        float hv = 0.f, lv = 0.f;
-        if (on) {
-          const double v = sd[2 * at(i, j) + comp];
-          const uint64_t bv = fpconv::bits64(v);
-          const uint64_t bw = fpconv::bits64(sd[2 * at(j, i) + comp]) ^ flip;
-          herm &= (bv == bw) || ((bv | bw) << 1) == 0;
-          fpconv::split_f64(v, hv, lv);
-          if (diag_owner && j == i) dtr = v;
+      for (int k = 0; k < kC / 2; ++k) {
+        float hv[2] = {0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int j = j0 + 2 * k + e;
+          float lv = 0.f;
+          if (on) {
+            const double v = sd[2 * pos(i, j) + comp];
+            const uint64_t bv = fpconv::bits64(v);
+            const uint64_t bw = fpconv::bits64(sd[2 * pos(j, i) + comp]) ^ flip;
+            herm &= (bv == bw) || ((bv | bw) << 1) == 0;
+            fpconv::split_f64(v, hv[e], lv);
+            if (diag_owner && j == i) dtr = v;
+          }
+          S.rlo[(2 * k + e) * 128 + t] = lv;
         }
-        rho[jj] = hv;
-        acc[jj] = 0.f;
-        S.rlo[jj * 128 + t] = lv;
+        rho[k] = x2::pack(hv[0], hv[1]);
+        acc[k] = 0;
       }
       if (on && h == 0)
         for (int j = 0; j < kW; ++j) {   // the whole row, in column order
           float hv, lv;
-          fpconv::split_f64(sd[2 * at(i, j) + comp], hv, lv);
+          fpconv::split_f64(sd[2 * pos(i, j) + comp], hv, lv);
           fro = __fmaf_rn(hv, hv, fro);
         }
     }
@@ -1102,11 +1135,12 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
     float mx = 0.f;
     float rho_d = 0.f, acc_d = 0.f, rs_d = 0.f;
 #pragma unroll
+    for (int k = 0; k < kC / 2; ++k) rho[k] = x2::mul(rho[k], x2::both(bsign));
+#pragma unroll
     for (int jj = 0; jj < kC; ++jj) {
-      rho[jj] *= bsign;
       S.rlo[jj * 128 + t] *= bsign;
-      mx = fmaxf(mx, fabsf(rho[jj]));
-      if (diag_owner && j0 + jj == i) rho_d = rho[jj];
+      mx = fmaxf(mx, fabsf(at(rho, jj)));
+      if (diag_owner && j0 + jj == i) rho_d = at(rho, jj);
     }
     if (!herm) flags |= LIME_FLAG_NOT_HERMITIAN;
     rs_d = rho_d;
@@ -1124,7 +1158,7 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
       const float magic = row_magic(row_bound());
       float dummy = 0.f;
 #pragma unroll
-      for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 8 * c, magic, dummy);
+      for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 4 * c, magic, dummy);
     }
     bool tr_pending = false;
     auto trace_check = [&]() {
@@ -1200,9 +1234,13 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
         }
         float nmx = 0.f;
         if (on) {
-          float u[kC];
+          uint64_t u[kC / 2];
 #pragma unroll
-          for (int jj = 0; jj < kC; ++jj) u[jj] = __fmaf_rn(tsign, xcol[(j0 + jj) * kLd], own[jj]);
+          for (int k = 0; k < kC / 2; ++k) {
+            const int j = j0 + 2 * k;
+            u[k] = x2::fma(x2::both(tsign), x2::pack(xcol[j * kLd], xcol[(j + 1) * kLd]),
+                           x2::pack(own[2 * k], own[2 * k + 1]));
+          }
           if (s < 3) {
             const float cst = (s == 2) ? a.c_full : a.c_half;
             const float wgt = (s == 0) ? 1.f : 2.f;
@@ -1213,12 +1251,12 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
               rs_d = __fmaf_rn(cst, ud, rho_d);
             }
 #pragma unroll
-            for (int jj = 0; jj < kC; ++jj) {
-              acc[jj] = __fmaf_rn(wgt, u[jj], acc[jj]);
-              u[jj] = __fmaf_rn(cst, u[jj], rho[jj]);
+            for (int k = 0; k < kC / 2; ++k) {
+              acc[k] = x2::fma(x2::both(wgt), u[k], acc[k]);
+              u[k] = x2::fma(x2::both(cst), u[k], rho[k]);
             }
 #pragma unroll
-            for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, u + 8 * c, magic, nmx);
+            for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, u + 4 * c, magic, nmx);
           } else {
             if (diag_owner) {
               const float xd = xrow[i];
@@ -1228,14 +1266,15 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
               rs_d = rho_d;
             }
 #pragma unroll
-            for (int jj = 0; jj < kC; ++jj) {
-              float lo = S.rlo[jj * 128 + t];
-              rho[jj] = rk4_final_f32(rho[jj], acc[jj], u[jj], a.c_sixth, a.c_sixth_lo, lo);
-              S.rlo[jj * 128 + t] = lo;
-              acc[jj] = 0.f;
+            for (int k = 0; k < kC / 2; ++k) {
+              float* const l = S.rlo + 2 * k * 128 + t;
+              uint64_t lo = x2::pack(l[0], l[128]);
+              rho[k] = rk4_final_f32x2(rho[k], acc[k], u[k], x2::both(a.c_sixth), x2::both(a.c_sixth_lo), lo);
+              x2::unpack(lo, l[0], l[128]);
+              acc[k] = 0;
             }
 #pragma unroll
-            for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 8 * c, magic, nmx);
+            for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 4 * c, magic, nmx);
           }
         }
         S.smax[(g + 1) & 1][t] = nmx;
@@ -1275,11 +1314,11 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
                     const double2 ev = E[(int64_t)j * n + i];   // E[j][i]
                     const float er = (float)ev.x, ei = (float)ev.y;
                     if (is_re) {
-                      pr = __fmaf_rn(er, rho[jj], pr);
-                      pi = __fmaf_rn(ei, rho[jj], pi);
+                      pr = __fmaf_rn(er, at(rho, jj), pr);
+                      pi = __fmaf_rn(ei, at(rho, jj), pi);
                     } else {
-                      pr = __fmaf_rn(ei, rho[jj], pr);
-                      pi = __fmaf_rn(-er, rho[jj], pi);
+                      pr = __fmaf_rn(ei, at(rho, jj), pr);
+                      pi = __fmaf_rn(-er, at(rho, jj), pi);
                     }
                   }
                 }
@@ -1318,9 +1357,9 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
       const uint64_t neg = is_re ? 0ull : 0x8000000000000000ull;
 #pragma unroll
       for (int jj = 0; jj < kC; ++jj) {
-        const double v = fpconv::scale_pow2(fpconv::widen_f32(rho[jj]) + fpconv::widen_f32(S.rlo[jj * 128 + t]), ebi);
-        if (!isfinite(rho[jj])) flags |= LIME_FLAG_NONFINITE;
-        sd[2 * at(i, j0 + jj) + comp] = fpconv::from_bits64(fpconv::bits64(v) ^ neg);
+        const double v = fpconv::scale_pow2(fpconv::widen_f32(at(rho, jj)) + fpconv::widen_f32(S.rlo[jj * 128 + t]), ebi);
+        if (!isfinite(at(rho, jj))) flags |= LIME_FLAG_NONFINITE;
+        sd[2 * pos(i, j0 + jj) + comp] = fpconv::from_bits64(fpconv::bits64(v) ^ neg);
       }
     }
     __syncthreads();
@@ -1328,7 +1367,7 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
       double2* out = a.rho_out + (int64_t)b * n * n;
       for (int e = t; e < n * n; e += Sh::kThreads) {
         const int ii = e / n, jj = e - ii * n;
-        if (in_bounds(((size_t)b * n * n + e) * 16, 16, a.rho_elems * 16, a.status)) out[e] = stg[at(ii, jj)];
+        if (in_bounds(((size_t)b * n * n + e) * 16, 16, a.rho_elems * 16, a.status)) out[e] = stg[pos(ii, jj)];
       }
     }
     __syncthreads();   // smax / rlo of this instance are no longer read
@@ -1560,7 +1599,7 @@ extern "C" int lime_lindblad_rk4_split(const LimeLindbladSplitDesc* d, void* str
   }
   // Dimensions up to 32 without a drive leave the 64-wide kernel, whose time
   // does not depend on n (20 steps of 16 instances 0.35 ms, of 4096 4.7 ms; at
-  // n = 16 0.17 and 0.72, at n = 32 0.21 and 1.40 ms).  One wait a stage
+  // n = 16 0.17 and 0.69, at n = 32 0.21 and 1.36 ms).  One wait a stage
   // (kDual) while its CTAs hold the batch in one round; beyond that the other
   // form holds twice as many (n = 32, 608 instances in one round: 0.27 ms,
   // where 304 in one round of the first take 0.22).
