@@ -632,24 +632,36 @@ __global__ void final_state_kernel(const float* Phi, const float* Plo, int Dp, i
 // (columns j < Rq real parts, Rq + j imaginary parts), operands Sr, Si and
 // Sr + Si as separate real B operands ([Rq/128][Dp/64] pieces each).
 
-// A pieces of row `row` of a real part of L (transposed = 0) or of the
-// observables (transposed = 1, element (o, a n + b) = E_o[b][a]): comp 0 the
-// real part, 1 the imaginary part, 2 their sum (formed in FP64).
-__global__ void convert_real_rows_kernel(const double2* M, int transposed, int comp, int n, int rows, int D, int KC,
-                                         uint8_t* A0, uint8_t* A1, uint8_t* A2, float* row_inv) {
+// A pieces of row `row` of the three real parts of L (transposed = 0) or of
+// the observables (transposed = 1, element (o, a n + b) = E_o[b][a]): real
+// part, imaginary part, and their sum (formed in FP64).  One pass for all
+// three, the source being the larger part of the traffic: the rows of a
+// 9216-dimensional generator 2.5 -> 2.1 ms.
+struct ThreeParts {
+  sg::APieces part[3];
+};
+__global__ void __launch_bounds__(256) convert_real_rows_kernel(const double2* M, int transposed, int n, int rows,
+                                                                int D, int KC, ThreeParts out) {
   const int row = blockIdx.x;
-  auto value = [&](int kk) -> double {
-    if (kk >= D) return 0.0;
-    double2 z;
-    if (transposed == 0) {
-      z = M[(size_t)row * D + kk];
-    } else {
-      const int ia = kk / n, ib = kk - ia * n;
-      z = M[(size_t)row * D + (size_t)ib * n + ia];
+  const auto entries = [&](int k, double (&x)[3][8]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int kk = k + i;
+      double2 z = cz();
+      if (kk < D) {
+        if (transposed == 0) {
+          z = M[(size_t)row * D + kk];
+        } else {
+          const int ia = kk / n, ib = kk - ia * n;
+          z = M[(size_t)row * D + (size_t)ib * n + ia];
+        }
+      }
+      x[0][i] = z.x;
+      x[1][i] = z.y;
+      x[2][i] = z.x + z.y;
     }
-    return comp == 0 ? z.x : (comp == 1 ? z.y : z.x + z.y);
   };
-  sg::convert_row_values(value, row, row < rows, KC * sg::kCK, KC, A0, A1, A2, row_inv);
+  sg::convert_row_parts<3>(entries, row, row < rows, KC * sg::kCK, KC, out.part);
 }
 
 struct Stage3 {
@@ -984,18 +996,19 @@ extern "C" int lime_redfield_rk4_split3(const LimeRedfieldSplitDesc* d, void* st
   for (int p = 0; p < 3; ++p) rinvE[p] = rows + (size_t)3 * MT * 128 + (size_t)p * MTo * 128;
   int64_t launches = 0;
 
+  rsp::ThreeParts tl, te;
   for (int p = 0; p < 3; ++p) {
-    rsp::convert_real_rows_kernel<<<Dp, 256, 0, st>>>(reinterpret_cast<const double2*>(d->R), 0, p, d->n, D, D, KC3,
-                                                     AL[p][0], AL[p][1], AL[p][2], rinvL[p]);
+    tl.part[p] = {{AL[p][0], AL[p][1], AL[p][2]}, rinvL[p]};
+    te.part[p] = {{AE[p][0], AE[p][1], AE[p][2]}, rinvE[p]};
+  }
+  rsp::convert_real_rows_kernel<<<Dp, 256, 0, st>>>(reinterpret_cast<const double2*>(d->R), 0, d->n, D, D, KC3, tl);
+  LIME_CUDA_TRY(cudaGetLastError());
+  ++launches;
+  if (MTo > 0) {
+    rsp::convert_real_rows_kernel<<<MTo * 128, 256, 0, st>>>(reinterpret_cast<const double2*>(d->obs_ops), 1, d->n,
+                                                            d->n_obs, D, KC3, te);
     LIME_CUDA_TRY(cudaGetLastError());
     ++launches;
-    if (MTo > 0) {
-      rsp::convert_real_rows_kernel<<<MTo * 128, 256, 0, st>>>(reinterpret_cast<const double2*>(d->obs_ops), 1, p,
-                                                              d->n, d->n_obs, D, KC3, AE[p][0], AE[p][1],
-                                                              AE[p][2], rinvE[p]);
-      LIME_CUDA_TRY(cudaGetLastError());
-      ++launches;
-    }
   }
   const int obs_every = d->obs_every > 0 ? d->obs_every : 1;
   if (MTo > 0) {

@@ -581,8 +581,8 @@ __device__ __forceinline__ bool seq_drain(Smem& S, const Tile& T, Seq& q) {
 }
 
 // ---------------------------------------------------------------- operand conversion
-// A pieces of one row of a real operand whose K entries are value(k), k in
-// [0, Ktot) (zero where the operand is padded).  The row is scaled by the
+// A pieces of one row of a real operand with Ktot entries (zero where the
+// operand is padded).  The row is scaled by the
 // power of two that brings its largest entry into [2^12, 2^13) and split as
 // A0 = 64 k (|k| <= 127) + fp16 residuals A1, A2; row_inv gets the inverse
 // scale (0 for padding rows and all-zero rows).  KC: chunks per row tile.
@@ -590,57 +590,82 @@ __device__ __forceinline__ bool seq_drain(Smem& S, const Tile& T, Seq& q) {
 // The FP64 pipe takes a warp's instruction every 64 clocks, and an entry cost
 // some fifteen of them, so the entries are split in integer and fp32
 // arithmetic (fpconv::split_a); eight consecutive entries a thread, 16-byte stores.
-// The rows of a 9216-dimensional generator (three real parts): 8.7 -> 2.6 ms; those
-// of 192 uneven chains with three dense operators: 1.58 -> 0.44 ms.
+// The rows of a 9216-dimensional generator (three real parts): 8.7 -> 2.1 ms; those
+// of 192 uneven chains with three dense operators: 1.58 -> 0.46 ms.
 
 __device__ __forceinline__ uint32_t pack_h2(__half a, __half b) {
   return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
 }
 
-template <class Val>
-__device__ __forceinline__ void convert_row_values(const Val& value, int row, bool valid, int Ktot, int KC,
-                                                   uint8_t* A0, uint8_t* A1, uint8_t* A2, float* row_inv) {
-  __shared__ unsigned long long red[32];
+// Where the pieces of an operand and its row scales go.
+struct APieces {
+  uint8_t* p[3];
+  float* row_inv;
+};
+
+// kParts real operands from one pass over their common source: entries(k,
+// v) gives the kParts values of eight consecutive entries k..k+7.
+template <int kParts, class Entries>
+__device__ __forceinline__ void convert_row_parts(const Entries& entries, int row, bool valid, int Ktot, int KC,
+                                                  const APieces (&out)[kParts]) {
+  __shared__ unsigned long long red[kParts][32];
   const unsigned long long inf = 0x7FF0000000000000ull;
+  const int nw = blockDim.x >> 5;
   // the largest |entry| by its bits; a NaN does not take part
-  unsigned long long mx = 0;
+  unsigned long long mx[kParts] = {};
+  double x[kParts][8];
   if (valid)
-    for (int k = threadIdx.x; k < Ktot; k += blockDim.x) {
-      const unsigned long long v = fpconv::bits64(value(k)) & ~(1ull << 63);
-      if (v <= inf && v > mx) mx = v;
+    for (int k = threadIdx.x * 8; k < Ktot; k += blockDim.x * 8) {
+      entries(k, x);
+#pragma unroll
+      for (int p = 0; p < kParts; ++p)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const unsigned long long v = fpconv::bits64(x[p][i]) & ~(1ull << 63);
+          if (v <= inf && v > mx[p]) mx[p] = v;
+        }
     }
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
-    mx = v > mx ? v : mx;
+  int sh[kParts];
+  bool live[kParts];
+#pragma unroll
+  for (int p = 0; p < kParts; ++p) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx[p], o);
+      mx[p] = v > mx[p] ? v : mx[p];
+    }
+    if ((threadIdx.x & 31) == 0) red[p][threadIdx.x >> 5] = mx[p];
   }
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
-  mx = red[0];
-  for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = red[w] > mx ? red[w] : mx;
-  const int sh = 12 + 1023 - (int)(mx >> 52);          // mx * 2^sh in [2^12, 2^13); a subnormal mx is too small below
-  const bool live = valid && mx != 0 && mx < inf && sh <= 140 && sh >= -140;
-  if (threadIdx.x == 0) row_inv[row] = live ? ldexpf(1.f, -sh) : 0.f;
+#pragma unroll
+  for (int p = 0; p < kParts; ++p) {
+    mx[p] = red[p][0];
+    for (int w = 1; w < nw; ++w) mx[p] = red[p][w] > mx[p] ? red[p][w] : mx[p];
+    sh[p] = 12 + 1023 - (int)(mx[p] >> 52);   // mx * 2^sh in [2^12, 2^13); a subnormal mx is too small below
+    live[p] = valid && mx[p] != 0 && mx[p] < inf && sh[p] <= 140 && sh[p] >= -140;
+    if (threadIdx.x == 0) out[p].row_inv[row] = live[p] ? ldexpf(1.f, -sh[p]) : 0.f;
+  }
   for (int k = threadIdx.x * 8; k < Ktot; k += blockDim.x * 8) {
-    uint32_t p0[4] = {0, 0, 0, 0}, p1[4] = {0, 0, 0, 0}, p2[4] = {0, 0, 0, 0};
-    if (live) {
-      double x[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = value(k + i);
-#pragma unroll
-      for (int i = 0; i < 8; i += 2) {
-        float va, vb;
-        __half a1, a2, b1, b2;
-        fpconv::split_a(fpconv::scale_pow2(x[i], sh), va, a1, a2);
-        fpconv::split_a(fpconv::scale_pow2(x[i + 1], sh), vb, b1, b2);
-        p0[i / 2] = pack_h2(__float2half_rn(va), __float2half_rn(vb));
-        p1[i / 2] = pack_h2(a1, b1);
-        p2[i / 2] = pack_h2(a2, b2);
-      }
-    }
+    if (valid && Ktot > (int)blockDim.x * 8) entries(k, x);   // else a thread's entries are still here
     const size_t off = piece_off(KC, row, k);
-    *reinterpret_cast<uint4*>(A0 + off) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
-    *reinterpret_cast<uint4*>(A1 + off) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
-    *reinterpret_cast<uint4*>(A2 + off) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+#pragma unroll
+    for (int p = 0; p < kParts; ++p) {
+      uint32_t p0[4] = {0, 0, 0, 0}, p1[4] = {0, 0, 0, 0}, p2[4] = {0, 0, 0, 0};
+      if (live[p]) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+          float va, vb;
+          __half a1, a2, b1, b2;
+          fpconv::split_a(fpconv::scale_pow2(x[p][i], sh[p]), va, a1, a2);
+          fpconv::split_a(fpconv::scale_pow2(x[p][i + 1], sh[p]), vb, b1, b2);
+          p0[i / 2] = pack_h2(__float2half_rn(va), __float2half_rn(vb));
+          p1[i / 2] = pack_h2(a1, b1);
+          p2[i / 2] = pack_h2(a2, b2);
+        }
+      }
+      *reinterpret_cast<uint4*>(out[p].p[0] + off) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+      *reinterpret_cast<uint4*>(out[p].p[1] + off) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+      *reinterpret_cast<uint4*>(out[p].p[2] + off) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
+    }
   }
 }
 
@@ -650,13 +675,17 @@ __device__ __forceinline__ void convert_row_values(const Val& value, int row, bo
 template <class Elem>
 __device__ __forceinline__ void convert_row(const Elem& elem, int row, bool valid, int cols, int Kp, int KC,
                                             uint8_t* A0, uint8_t* A1, uint8_t* A2, float* row_inv) {
-  auto value = [&](int k) -> double {
-    const int kk = k < Kp ? k : k - Kp;
-    if (kk >= cols) return 0.0;
-    const double2 z = elem(kk);
-    return k < Kp ? z.x : z.y;
+  const auto entries = [&](int k, double (&x)[1][8]) {
+    const bool im = k >= Kp;   // (Kp is a multiple of 8)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int kk = (im ? k - Kp : k) + i;
+      const double2 z = kk < cols ? elem(kk) : make_double2(0.0, 0.0);
+      x[0][i] = im ? z.y : z.x;
+    }
   };
-  convert_row_values(value, row, valid, 2 * Kp, KC, A0, A1, A2, row_inv);
+  const APieces out[1] = {{{A0, A1, A2}, row_inv}};
+  convert_row_parts<1>(entries, row, valid, 2 * Kp, KC, out);
 }
 
 }  // namespace sg
