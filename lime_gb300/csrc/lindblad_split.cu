@@ -318,15 +318,22 @@ __device__ __forceinline__ double a_elem_scaled(const double2* heff, int n, int 
 // the FP64 instructions, so the pieces are those of the kernel's own split.
 // For the stand-alone preparation kernel, whose time is otherwise the FP64
 // pipe's (a few operations per clock per SM on this part).
-__device__ __forceinline__ float a_row_max_int(const double2* heff, int n, int i, bool xi_row, int ea) {
-  float m = 0.f;
-#pragma unroll 4
-  for (int k = 0; k < 128; ++k) {
-    float hi, lo;
-    fpconv::split_f64(a_elem_scaled(heff, n, i, k, xi_row, ea), hi, lo);
-    m = fmaxf(m, fabsf(hi));
+__device__ __forceinline__ float a_row_max_int(const double2* heff, int ld, int i, int ea) {
+  // the largest entry by its bits (a NaN does not take part), converted once:
+  // scaling and rounding keep the order.  Both rows of site i hold the same
+  // 64 complex entries.
+  uint64_t m = 0;
+#pragma unroll 8
+  for (int k = 0; k < kN; ++k) {
+    const double2 z = heff[(int64_t)i * ld + k];
+    const uint64_t u = fpconv::bits64(z.x) & ~(1ull << 63), v = fpconv::bits64(z.y) & ~(1ull << 63);
+    if (u <= 0x7FF0000000000000ull && u > m) m = u;
+    if (v <= 0x7FF0000000000000ull && v > m) m = v;
   }
-  return m;
+  if (m == 0) return 0.f;
+  float hi, lo;
+  fpconv::split_f64(fpconv::scale_pow2(fpconv::from_bits64(m), ea), hi, lo);
+  return hi;
 }
 
 __device__ __forceinline__ void a_pieces_row_int(const double2* heff, int n, int i, bool xi_row, int h, int qq,
@@ -375,7 +382,7 @@ __global__ void __launch_bounds__(kThreads) prepare_a_kernel(const double2* heff
   }
   __syncthreads();
   float magic, qmax;
-  a_row_quantum(a_row_max_int(hs, kPrepLd, i, xi_row, ea), magic, qmax);
+  a_row_quantum(a_row_max_int(hs, kPrepLd, i, ea), magic, qmax);
 #pragma unroll 1
   for (int qq = 0; qq < 2; ++qq) {
     uint32_t p[3][16];
