@@ -312,15 +312,17 @@ __global__ void __launch_bounds__(sg::kThreads, 1) gemm_kernel(Args a) {
 // tiles j, j + gridDim.x, ... of the concatenated tile list, whose groups
 // the host orders by decreasing chunks per tile (largest tiles first).
 constexpr int kMaxGroups = 16;
-struct Groups {
+template <int kMax>
+struct GroupsOf {
   int n_groups, n_items;
-  int start[kMaxGroups + 1];          // first tile of each group in the list
-  Args g[kMaxGroups];
+  int start[kMax + 1];                // first tile of each group in the list
+  Args g[kMax];
 };
+using Groups = GroupsOf<kMaxGroups>;
 static_assert(sizeof(Groups) <= 30000, "kernel parameter space");
 
-template <bool kZ>
-__global__ void __launch_bounds__(sg::kThreads, 1) gemm_groups_kernel(const __grid_constant__ Groups m) {
+template <bool kZ, int kMax>
+__global__ void __launch_bounds__(sg::kThreads, 1) gemm_groups_kernel(const __grid_constant__ GroupsOf<kMax> m) {
   extern __shared__ uint8_t smem_raw[];
   sg::Smem& S = *reinterpret_cast<sg::Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   sg::setup(S);
@@ -1056,6 +1058,38 @@ int lsm_prepare(const LimeLindbladStreamDesc* d, LsmRun& r, cudaStream_t st, int
   return K > 0 ? LIME_OK : zero_padding(L, d->n, r.B1[1][0], r.B1[1][1], st);
 }
 
+// The GEMM 1 or GEMM 2 tiles of one propagation: a CTA each, or, when there
+// are more than the SMs hold at once, the persistent sequence of the grouped
+// launch, whose CTAs load and multiply the next tile during the epilogue of
+// the last (384 tiles of 129 levels, 2.5 rounds: 43.4 -> 35.8 us).
+template <bool kZ>
+int lsm_gemm(const lsm::Args& a, int tiles, int sms, cudaStream_t st) {
+  const size_t smem = sg::kSmemBytes;
+  if (tiles <= sms) {
+    LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<kZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    lsm::gemm_kernel<kZ><<<tiles, sg::kThreads, smem, st>>>(a);
+  } else {
+    lsm::GroupsOf<1> m;
+    m.n_groups = 1;
+    m.n_items = tiles;
+    m.start[0] = 0;
+    m.start[1] = tiles;
+    m.g[0] = a;
+    auto kern = lsm::gemm_groups_kernel<kZ, 1>;
+    LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<sms, sg::kThreads, smem, st>>>(m);
+  }
+  LIME_CUDA_TRY(cudaGetLastError());
+  return LIME_OK;
+}
+
+int lsm_sms(int& sms) {
+  int dev = 0;
+  LIME_CUDA_TRY(cudaGetDevice(&dev));
+  LIME_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return LIME_OK;
+}
+
 int lsm_zlower_grid(const lsm::Args& a, int B) {
   const int xbs = a.np / 128;
   const size_t runs = (size_t)B * 2 * (xbs * (xbs - 1) / 2) * 128 * 16;
@@ -1111,9 +1145,8 @@ extern "C" int lime_lindblad_rk4_stream(const LimeLindbladStreamDesc* d, void* s
   const int B = r.B, K = r.K, G = r.G;
   lsm::Args& a = r.a;
   const int tb = B * lsm::state_tiles(d->n) * lsm::state_tiles(d->n);
-  const size_t smem = sg::kSmemBytes;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int sms = 0, grc = lsm_sms(sms);
+  if (grc != LIME_OK) return grc;
   int cur = 0;
   for (int step = 0; step < d->n_steps; ++step) {
     if (d->n_drive > 0) {
@@ -1131,13 +1164,13 @@ extern "C" int lime_lindblad_rk4_stream(const LimeLindbladStreamDesc* d, void* s
     }
     for (int s = 0; s < 4; ++s) {
       lsm_bind_stage(r, s, cur);
-      lsm::gemm_kernel<false><<<B * L.MT1 * L.NT, sg::kThreads, smem, st>>>(a);
-      LIME_CUDA_TRY(cudaGetLastError());
+      grc = lsm_gemm<false>(a, B * L.MT1 * L.NT, sms, st);
+      if (grc != LIME_OK) return grc;
       ++launches;
       if (K > 0) {
-        lsm::gemm_kernel<true><<<B * lsm::gemm2_tiles(a), sg::kThreads, smem, st>>>(a);
+        grc = lsm_gemm<true>(a, B * lsm::gemm2_tiles(a), sms, st);
+        if (grc != LIME_OK) return grc;
         if (a.zhalf) {
-          LIME_CUDA_TRY(cudaGetLastError());
           lsm::zlower_kernel<<<lsm_zlower_grid(a, B), 256, 0, st>>>(a, B);
           ++launches;
         }
@@ -1181,9 +1214,9 @@ extern "C" int lime_lindblad_rk4_stream_groups(const LimeLindbladStreamDesc* des
   LIME_CUDA_TRY(cudaGetDevice(&dev));
   LIME_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const size_t smem = sg::kSmemBytes;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<false, lsm::kMaxGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<true, lsm::kMaxGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   // tile lists: groups by decreasing chunks per tile (order 1), or as given (order 0)
   int ord1[lsm::kMaxGroups], ord2[lsm::kMaxGroups];
@@ -1224,12 +1257,12 @@ extern "C" int lime_lindblad_rk4_stream_groups(const LimeLindbladStreamDesc* des
     for (int s = 0; s < 4; ++s) {
       for (int i = 0; i < n_groups; ++i) lsm_bind_stage(runs[i], s, cur);
       fill(m1, ord1, n_groups, false);
-      lsm::gemm_groups_kernel<false><<<grid_of(m1.n_items), sg::kThreads, smem, st>>>(m1);
+      lsm::gemm_groups_kernel<false, lsm::kMaxGroups><<<grid_of(m1.n_items), sg::kThreads, smem, st>>>(m1);
       LIME_CUDA_TRY(cudaGetLastError());
       ++launches;
       if (n2 > 0) {
         fill(m2, ord2, n2, true);
-        lsm::gemm_groups_kernel<true><<<grid_of(m2.n_items), sg::kThreads, smem, st>>>(m2);
+        lsm::gemm_groups_kernel<true, lsm::kMaxGroups><<<grid_of(m2.n_items), sg::kThreads, smem, st>>>(m2);
         LIME_CUDA_TRY(cudaGetLastError());
         ++launches;
         for (int i = 0; i < n_groups; ++i) {
@@ -1358,8 +1391,8 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
   LIME_CUDA_TRY(cudaMemsetAsync(J.lmax, 0, 8, st));          // lmax and sl_exp
   const int zrc = zero_padding(L, d->n, B1[1][0], B1[1][1], st);
   if (zrc != LIME_OK) return zrc;
-  const size_t smem = sg::kSmemBytes;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int sms = 0, grc = lsm_sms(sms);
+  if (grc != LIME_OK) return grc;
   const size_t runs = (size_t)B * L.W * (L.np / 8);
   const int eb = (int)((runs + 255) / 256 < 65535 ? (runs + 255) / 256 : 65535);
   const int tb = B * lsm::state_tiles(d->n) * lsm::state_tiles(d->n);
@@ -1387,8 +1420,8 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
         af.Sc = Sbuf[cur];
         af.Sn = Sbuf[cur ^ 1];
         af.stage_store = store + ((size_t)s * 4 + k) * B * inst;
-        lsm::gemm_kernel<false><<<gemm_grid, sg::kThreads, smem, st>>>(af);
-        LIME_CUDA_TRY(cudaGetLastError());
+        grc = lsm_gemm<false>(af, gemm_grid, sms, st);
+        if (grc != LIME_OK) return grc;
         lsm::finish_kernel<<<tb, 256, 0, st>>>(af);
         LIME_CUDA_TRY(cudaGetLastError());
         launches += 2;
@@ -1418,8 +1451,8 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
         aa.Sc = Sbuf[c];
         aa.B1n[0] = B1[c ^ 1][0]; aa.B1n[1] = B1[c ^ 1][1];
         aa.Sn = Sbuf[c ^ 1];
-        lsm::gemm_kernel<false><<<gemm_grid, sg::kThreads, smem, st>>>(aa);
-        LIME_CUDA_TRY(cudaGetLastError());
+        grc = lsm_gemm<false>(aa, gemm_grid, sms, st);
+        if (grc != LIME_OK) return grc;
         lsm::adj_grad_kernel<<<B * ((d->n + 7) / 8), lsm::kGradThreads, 0, st>>>(
             aa, Sbuf[c], store + ((size_t)s * 4 + (i - 1)) * B * inst, d->grad_diag, d->grad_bond, d->grad_gamma);
         LIME_CUDA_TRY(cudaGetLastError());
