@@ -90,6 +90,15 @@ __device__ __forceinline__ float rk4_final_f32(float x, float acc, float f, floa
   return hi2;
 }
 
+// ---------------------------------------------------------------- launches in a chain
+// Programmatic dependent launch: a kernel of a chain of short ones is set up
+// before the one before it has ended, and waits for that here, before its
+// first access to global memory.  (An early launch_dependents makes the long
+// chains slower: the waiting CTAs hold the SMs of the kernel's tail.)
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 }  // namespace lime
 
 #define LIME_CUDA_TRY(expr)                            \
@@ -97,3 +106,31 @@ __device__ __forceinline__ float rk4_final_f32(float x, float acc, float f, floa
     cudaError_t _e = (expr);                           \
     if (_e != cudaSuccess) return LIME_ERR_CUDA;       \
   } while (0)
+
+#define LIME_TRY(expr)                                 \
+  do {                                                 \
+    const int _rc = (expr);                            \
+    if (_rc != LIME_OK) return _rc;                    \
+  } while (0)
+
+namespace lime {
+
+// Launch of a kernel that calls chain_wait.
+template <class... P, class... A>
+inline int launch_chained(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                          const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  LIME_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+  return LIME_OK;
+}
+
+}  // namespace lime

@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(sg::kThreads, 1) gemm_kernel(Args a) {
   extern __shared__ uint8_t smem_raw[];
   sg::Smem& S = *reinterpret_cast<sg::Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   sg::setup(S);
+  chain_wait();
   sg::Tile T;
   int b, mt, nt;
   gemm_tile_of<kZ>(a, blockIdx.x, T, b, mt, nt);
@@ -326,6 +327,7 @@ __global__ void __launch_bounds__(sg::kThreads, 1) gemm_groups_kernel(const __gr
   extern __shared__ uint8_t smem_raw[];
   sg::Smem& S = *reinterpret_cast<sg::Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   sg::setup(S);
+  chain_wait();
   sg::Seq q;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   auto group_of = [&](int item) {
@@ -416,6 +418,7 @@ __device__ __forceinline__ TileItem load_tile_item(const Args& a, float (*T)[32]
 
 // The stage update without dense operators (no GEMM 2).
 __global__ void __launch_bounds__(256) finish_kernel(Args a) {
+  chain_wait();
   __shared__ float T[2][32][33];
   const TileItem it = load_tile_item(a, T);
   if (!it.live) return;
@@ -438,6 +441,7 @@ __global__ void __launch_bounds__(256) finish_kernel(Args a) {
 // from the strictly upper tiles' raw Z in Zg, then f and the RK4 update as
 // in GEMM 2's epilogue.  One thread per run of 8 rows of one state column.
 __global__ void __launch_bounds__(256) zlower_kernel(Args a, int batch) {
+  chain_wait();
   const int np = a.np, xbs = np / 128;
   const int pairs = xbs * (xbs - 1) / 2;               // (mt, xb) with mt > xb
   const size_t per_inst = (size_t)2 * pairs * 128 * 16;  // components x pairs x columns x 8-row runs
@@ -586,6 +590,7 @@ __device__ __forceinline__ void add_term(double& sr, double& si, double2 e, doub
 }
 __global__ void __launch_bounds__(kObsThreads) observe_kernel(Args a, const double2* E, int64_t e_stride, int n_obs,
                                                               double2* out, int n_slots, int slot) {
+  chain_wait();
   const int b = blockIdx.x / n_obs, o = blockIdx.x % n_obs;
   const int per = a.n * a.n;
   const double2* Eo = E + (e_stride ? (int64_t)(b % a.P) * e_stride : 0) + (int64_t)o * per;
@@ -616,6 +621,7 @@ __global__ void __launch_bounds__(kObsThreads) observe_kernel(Args a, const doub
 // ([P|1][n_obs][n]): a warp each.
 __global__ void __launch_bounds__(128) observe_diag_kernel(Args a, const double2* E, int64_t e_stride, int n_obs,
                                                            int batch, double2* out, int n_slots, int slot) {
+  chain_wait();
   const int64_t w = blockIdx.x * (int64_t)4 + (threadIdx.x >> 5);
   const int b = (int)(w / n_obs), o = (int)(w % n_obs), lane = threadIdx.x & 31;
   if (b >= batch) return;
@@ -666,6 +672,7 @@ struct AdjState {
 // bound * max |lam| at 2^13 / 1.25 (lam changes by orders of magnitude over a
 // backward pass, one scale for all steps would waste the fixed-point range).
 __global__ void adj_scale_kernel(AdjState j) {
+  chain_wait();
   const float m = __uint_as_float(*j.lmax) * j.bound;
   int e = 0;
   if (m > 0.f && isfinite(m)) {
@@ -684,6 +691,7 @@ __global__ void adj_scale_kernel(AdjState j) {
 // coefficient pairs ([P|1][n_obs][component][x][row], two FMAs an element).
 __global__ void adj_source_kernel(Args a, AdjState j, int batch, const double2* E, int64_t e_stride, int n_obs,
                                   const double2* gsrc, int n_slots, int slot, const float2* Q) {
+  chain_wait();
   const size_t runs = (size_t)a.W * (a.np / 8);
   const size_t total = (size_t)batch * runs;
   float mx = 0.f;
@@ -750,6 +758,7 @@ __global__ void adj_source_kernel(Args a, AdjState j, int batch, const double2* 
 
 // ab_4 = dt/6 lam as the next GEMM 1 input (fp32 copy and scaled B pieces).
 __global__ void adj_start_kernel(Args a, AdjState j, int batch, float dt6) {
+  chain_wait();
   const size_t runs = (size_t)a.W * (a.np / 8);
   const size_t total = (size_t)batch * runs;
   const float sl = ldexpf(1.f, *j.sl_exp);
@@ -781,6 +790,7 @@ __global__ void adj_start_kernel(Args a, AdjState j, int batch, float dt6) {
 // yb_i = L^dag ab_i (Xg = G ab_i from GEMM 1, ab_i in Sc) and the next
 // adjoint stage input (stage i = 4, 3, 2) or the new lam (i = 1).
 __global__ void __launch_bounds__(256) adj_finish_kernel(Args a, AdjState j, int stage_i, float c_l, float c_y) {
+  chain_wait();
   __shared__ float T[2][32][33];
   const TileItem it = load_tile_item(a, T);
   if (!it.live) return;
@@ -837,6 +847,7 @@ __global__ void __launch_bounds__(256) adj_finish_kernel(Args a, AdjState j, int
 constexpr int kGradThreads = 128;
 __global__ void __launch_bounds__(kGradThreads) adj_grad_kernel(Args a, const float* ab, const float* yst, double* gd,
                                                                 double* gb, double* gg) {
+  chain_wait();
   const int runs = (a.n + 7) / 8;
   const int b = blockIdx.x / runs, k0 = (blockIdx.x % runs) * 8;
   const int n = a.n, np = a.np;
@@ -1067,7 +1078,7 @@ int lsm_gemm(const lsm::Args& a, int tiles, int sms, cudaStream_t st) {
   const size_t smem = sg::kSmemBytes;
   if (tiles <= sms) {
     LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_kernel<kZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    lsm::gemm_kernel<kZ><<<tiles, sg::kThreads, smem, st>>>(a);
+    LIME_TRY(launch_chained(lsm::gemm_kernel<kZ>, tiles, sg::kThreads, smem, st, a));
   } else {
     lsm::GroupsOf<1> m;
     m.n_groups = 1;
@@ -1077,7 +1088,7 @@ int lsm_gemm(const lsm::Args& a, int tiles, int sms, cudaStream_t st) {
     m.g[0] = a;
     auto kern = lsm::gemm_groups_kernel<kZ, 1>;
     LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<sms, sg::kThreads, smem, st>>>(m);
+    LIME_TRY(launch_chained(kern, sms, sg::kThreads, smem, st, m));
   }
   LIME_CUDA_TRY(cudaGetLastError());
   return LIME_OK;
@@ -1113,12 +1124,11 @@ int lsm_observe(const LimeLindbladStreamDesc* d, LsmRun& r, int step, cudaStream
     double2* out = reinterpret_cast<double2*>(d->obs_out);
     const int slots = d->n_steps / obs_every, slot = (step + 1) / obs_every - 1;
     if (d->obs_diag)
-      lsm::observe_diag_kernel<<<(unsigned)(((int64_t)r.B * d->n_obs + 3) / 4), 128, 0, st>>>(
-          r.a, E, d->obs_stride, d->n_obs, r.B, out, slots, slot);
+      LIME_TRY(launch_chained(lsm::observe_diag_kernel,
+                              (unsigned)(((int64_t)r.B * d->n_obs + 3) / 4), 128, 0, st, r.a, E, d->obs_stride, d->n_obs, r.B, out, slots, slot));
     else
-      lsm::observe_kernel<<<r.B * d->n_obs, lsm::kObsThreads, 0, st>>>(r.a, E, d->obs_stride, d->n_obs, out, slots,
-                                                                       slot);
-    LIME_CUDA_TRY(cudaGetLastError());
+      LIME_TRY(launch_chained(lsm::observe_kernel,
+                              r.B * d->n_obs, lsm::kObsThreads, 0, st, r.a, E, d->obs_stride, d->n_obs, out, slots, slot));
     ++launches;
   }
   return LIME_OK;
@@ -1171,11 +1181,11 @@ extern "C" int lime_lindblad_rk4_stream(const LimeLindbladStreamDesc* d, void* s
         grc = lsm_gemm<true>(a, B * lsm::gemm2_tiles(a), sms, st);
         if (grc != LIME_OK) return grc;
         if (a.zhalf) {
-          lsm::zlower_kernel<<<lsm_zlower_grid(a, B), 256, 0, st>>>(a, B);
+          LIME_TRY(launch_chained(lsm::zlower_kernel, lsm_zlower_grid(a, B), 256, 0, st, a, B));
           ++launches;
         }
       } else {
-        lsm::finish_kernel<<<tb, 256, 0, st>>>(a);
+        LIME_TRY(launch_chained(lsm::finish_kernel, tb, 256, 0, st, a));
       }
       LIME_CUDA_TRY(cudaGetLastError());
       ++launches;
@@ -1257,26 +1267,25 @@ extern "C" int lime_lindblad_rk4_stream_groups(const LimeLindbladStreamDesc* des
     for (int s = 0; s < 4; ++s) {
       for (int i = 0; i < n_groups; ++i) lsm_bind_stage(runs[i], s, cur);
       fill(m1, ord1, n_groups, false);
-      lsm::gemm_groups_kernel<false, lsm::kMaxGroups><<<grid_of(m1.n_items), sg::kThreads, smem, st>>>(m1);
-      LIME_CUDA_TRY(cudaGetLastError());
+      LIME_TRY(launch_chained(lsm::gemm_groups_kernel<false, lsm::kMaxGroups>, grid_of(m1.n_items), sg::kThreads,
+                              smem, st, m1));
       ++launches;
       if (n2 > 0) {
         fill(m2, ord2, n2, true);
-        lsm::gemm_groups_kernel<true, lsm::kMaxGroups><<<grid_of(m2.n_items), sg::kThreads, smem, st>>>(m2);
-        LIME_CUDA_TRY(cudaGetLastError());
+        LIME_TRY(launch_chained(lsm::gemm_groups_kernel<true, lsm::kMaxGroups>, grid_of(m2.n_items), sg::kThreads,
+                                smem, st, m2));
         ++launches;
         for (int i = 0; i < n_groups; ++i) {
           if (runs[i].K == 0 || !runs[i].a.zhalf) continue;
-          lsm::zlower_kernel<<<lsm_zlower_grid(runs[i].a, runs[i].B), 256, 0, st>>>(runs[i].a, runs[i].B);
-          LIME_CUDA_TRY(cudaGetLastError());
+          LIME_TRY(launch_chained(lsm::zlower_kernel, lsm_zlower_grid(runs[i].a, runs[i].B), 256, 0, st, runs[i].a,
+                                  runs[i].B));
           ++launches;
         }
       }
       for (int i = 0; i < n_groups; ++i) {
         if (runs[i].K > 0) continue;
         const int tb = runs[i].B * lsm::state_tiles(runs[i].a.n) * lsm::state_tiles(runs[i].a.n);
-        lsm::finish_kernel<<<tb, 256, 0, st>>>(runs[i].a);
-        LIME_CUDA_TRY(cudaGetLastError());
+        LIME_TRY(launch_chained(lsm::finish_kernel, tb, 256, 0, st, runs[i].a));
         ++launches;
       }
       cur ^= 1;
@@ -1422,8 +1431,7 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
         af.stage_store = store + ((size_t)s * 4 + k) * B * inst;
         grc = lsm_gemm<false>(af, gemm_grid, sms, st);
         if (grc != LIME_OK) return grc;
-        lsm::finish_kernel<<<tb, 256, 0, st>>>(af);
-        LIME_CUDA_TRY(cudaGetLastError());
+        LIME_TRY(launch_chained(lsm::finish_kernel, tb, 256, 0, st, af));
         launches += 2;
         cur ^= 1;
       }
@@ -1436,15 +1444,10 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
       const int slot = (d->n_obs > 0 && ((gstep + 1) % obs_every) == 0) ? (gstep + 1) / obs_every - 1 : -1;
       aa.B1n[0] = B1[c][0]; aa.B1n[1] = B1[c][1];
       aa.Sn = Sbuf[c];
-      lsm::adj_source_kernel<<<eb, 256, 0, st>>>(aa, J, B, reinterpret_cast<const double2*>(d->obs_ops),
-                                                  d->obs_stride, d->n_obs,
-                                                  reinterpret_cast<const double2*>(d->obs_grad), n_slots, slot,
-                                                  reinterpret_cast<const float2*>(d->obs_coef));
-      LIME_CUDA_TRY(cudaGetLastError());
-      lsm::adj_scale_kernel<<<1, 1, 0, st>>>(J);
-      LIME_CUDA_TRY(cudaGetLastError());
-      lsm::adj_start_kernel<<<eb, 256, 0, st>>>(aa, J, B, (float)(dt / 6.0));
-      LIME_CUDA_TRY(cudaGetLastError());
+      LIME_TRY(launch_chained(lsm::adj_source_kernel, eb, 256, 0, st, aa, J, B,
+                              reinterpret_cast<const double2*>(d->obs_ops), d->obs_stride, d->n_obs, reinterpret_cast<const double2*>(d->obs_grad), n_slots, slot, reinterpret_cast<const float2*>(d->obs_coef)));
+      LIME_TRY(launch_chained(lsm::adj_scale_kernel, 1, 1, 0, st, J));
+      LIME_TRY(launch_chained(lsm::adj_start_kernel, eb, 256, 0, st, aa, J, B, (float)(dt / 6.0)));
       launches += 3;
       for (int i = 4; i >= 1; --i) {
         aa.B1c[0] = B1[c][0]; aa.B1c[1] = B1[c][1];
@@ -1453,13 +1456,11 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
         aa.Sn = Sbuf[c ^ 1];
         grc = lsm_gemm<false>(aa, gemm_grid, sms, st);
         if (grc != LIME_OK) return grc;
-        lsm::adj_grad_kernel<<<B * ((d->n + 7) / 8), lsm::kGradThreads, 0, st>>>(
-            aa, Sbuf[c], store + ((size_t)s * 4 + (i - 1)) * B * inst, d->grad_diag, d->grad_bond, d->grad_gamma);
-        LIME_CUDA_TRY(cudaGetLastError());
+        LIME_TRY(launch_chained(lsm::adj_grad_kernel,
+                                B * ((d->n + 7) / 8), lsm::kGradThreads, 0, st, aa, Sbuf[c], store + ((size_t)s * 4 + (i - 1)) * B * inst, d->grad_diag, d->grad_bond, d->grad_gamma));
         const float c_l = (float)(i == 2 ? dt / 6.0 : dt / 3.0);
         const float c_y = (float)(i == 4 ? dt : dt / 2.0);
-        lsm::adj_finish_kernel<<<tb, 256, 0, st>>>(aa, J, i, c_l, c_y);
-        LIME_CUDA_TRY(cudaGetLastError());
+        LIME_TRY(launch_chained(lsm::adj_finish_kernel, tb, 256, 0, st, aa, J, i, c_l, c_y));
         launches += 3;
         if (i > 1) c ^= 1;
       }
