@@ -56,6 +56,7 @@ struct RK4Args {
   int n_drive;
   const double2* drive_ops;
   const double* drive_coef;
+  int b0;                 // first instance of the launch (the batch's pointers start there)
   // shared-memory plan (RK4Plan)
   int cluster, ld, vcap, row_cap, y_smem;
   // extents for the bounds-checked build (elements of obs_out and states)
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(kE == 1 ? kMaxThreads + 32 : kMaxThreads, 1) l
   const int b = kCg ? (int)(blockIdx.x / C) : (int)blockIdx.x;
   const int n = a.n, ld = a.ld;
   const int64_t nn = (int64_t)n * n;
-  const int p = b % a.param_batch;
+  const int p = (a.b0 + b) % a.param_batch;
   double2* rho = a.rho + b * nn;
   const double2* heff0 = a.heff + p * a.heff_stride;
   const double2* m = a.m ? a.m + p * a.m_stride : nullptr;
@@ -522,25 +523,14 @@ struct RK4Plan {
 
 constexpr size_t kSmemMax = 227 * 1024 - sizeof(Head) - 1024;
 
-// How one call is laid out.
-//  - cluster: the largest of 8, 4, 2 that keeps batch * cluster on the chip
-//    (the occupancy calculator finds room for 15, 36 and 76 clusters with one
-//    CTA a SM) and leaves every CTA `least` items.  Below that the L2 round
-//    trip and cluster barrier of a stage cost more than the FP64 work they
-//    divide; with dense operators the work an item carries is larger.
+// How a launch with clusters of c CTAs is laid out.
 //  - items a thread: the fewest of 1, 2, 4, 8 that 512 threads cover.
 //  - shared memory: the stage inputs, the generator's values as full rows if
 //    they fit, Y of up to four operators, the entry lists.
-static RK4Plan plan_rk4(int n, int batch, int k_dense) {
+static RK4Plan plan_rk4(int n, int c, int k_dense) {
   RK4Plan P{};
   const int64_t nn = (int64_t)n * n;
-  const int64_t least = k_dense > 0 ? 128 : 512;
-  P.cluster = 1;
-  for (int c = 8; c > 1; c >>= 1)
-    if (batch <= (c == 8 ? 15 : c == 4 ? 36 : 76) && nn >= c * least) {
-      P.cluster = c;
-      break;
-    }
+  P.cluster = c;
   const int64_t per = (nn + P.cluster - 1) / P.cluster;
   P.e = per <= kMaxThreads ? 1 : per <= 2 * kMaxThreads ? 2 : per <= 4 * kMaxThreads ? 4 : per <= 8 * kMaxThreads ? 8 : 0;
   if (n > 65535 || (P.cluster == 1 && n > 64)) P.e = 0;
@@ -570,6 +560,90 @@ static RK4Plan plan_rk4(int n, int batch, int k_dense) {
   }
   P.smem = (size_t)((int64_t)kSmemMax - left);
   return P;
+}
+
+// A batch runs as rounds of one CTA an instance while they fill the chip,
+// and what is left over (or a batch smaller than the chip) as launches of
+// clusters, one round each: kRoom[c] clusters of c CTAs with an SM each fit
+// at once (occupancy calculator; 152 SMs).  The split is the cheapest by this
+// count of a stage's clocks: 64 an FP64 instruction and warp of the busiest of
+// an SM's four partitions, plus the cluster's exchange through L2 (3000
+// measured, with the four barriers of dense operators 12000, against 600 for
+// a barrier of one CTA) and a launch's share.  Without dense operators the
+// entries of a row are not known here; 12 FP64 instructions an item stand for
+// a chain.  A cluster leaves every CTA at least 512 items (128 with dense
+// operators): below that the exchange costs more than it divides.
+// Measured against one launch with one cluster size (a power of two, and one
+// CTA an instance from 77 on), 37 levels with three dense operators: 170
+// instances, 6 steps, 16.1 -> 9.9 ms; 48, 20 steps, 14.3 -> 12.3; 64-site
+// chains, 160, 8 steps, 1.22 -> 0.89, 512, 8 steps, 2.20 -> 2.09.
+constexpr int kMaxCluster = 8;
+constexpr int kRoom[kMaxCluster + 1] = {0, 152, 76, 46, 36, 28, 23, 15, 15};
+
+static double stage_clocks(int n, int c, int k_dense) {
+  const RK4Plan P = plan_rk4(n, c, k_dense);
+  const int64_t nn = (int64_t)n * n, per = (nn + c - 1) / c, rows = (int64_t)k_dense * nn;
+  // instructions of the busiest partition for `work` thread items in rounds of the CTA's threads
+  const auto busiest = [&](int64_t work) {
+    return (double)(work / P.nt) * ((P.nt / 32 + 3) / 4) + (double)(((work % P.nt + 31) / 32 + 3) / 4);
+  };
+  const double item = busiest(per), y = busiest((rows + c - 1) / c);
+  return 64.0 * (item * (k_dense > 0 ? (4.0 + 2.0 * k_dense) * n : 12.0) + y * 4.0 * n) +
+         (c == 1 ? 600.0 : k_dense > 0 ? 12000.0 : 3000.0);
+}
+
+struct RK4Part {
+  int b0, count, cluster;
+};
+
+// parts of a batch, at most kMaxParts
+constexpr int kMaxParts = 4;
+static int split_batch(int n, int batch, int k_dense, int n_steps, RK4Part* out) {
+  const int64_t nn = (int64_t)n * n, least = k_dense > 0 ? 128 : 512;
+  double t[kMaxCluster + 1];
+  int most = 1;
+  for (int c = 1; c <= kMaxCluster && (c == 1 || nn >= c * least); ++c) {
+    t[c] = stage_clocks(n, c, k_dense) + 60000.0 / (4.0 * n_steps);
+    most = c;
+  }
+  // best[r]: cheapest rounds for r instances; a remainder of parts parts
+  const int room = kRoom[1], rest = batch % room, full = batch - rest;
+  double best[kMaxParts + 1][kRoom[1] + 1];
+  int pick[kMaxParts + 1][kRoom[1] + 1];
+  for (int k = 0; k <= kMaxParts; ++k)
+    for (int r = 0; r <= rest; ++r) {
+      best[k][r] = r == 0 ? 0.0 : 1e300;
+      pick[k][r] = 0;
+      if (k > 0 && r > 0)
+        for (int c = 1; c <= most; ++c) {
+          const double v = t[c] + best[k - 1][r > kRoom[c] ? r - kRoom[c] : 0];
+          if (v < best[k][r]) {
+            best[k][r] = v;
+            pick[k][r] = c;
+          }
+        }
+    }
+  // one launch for the remainder, unless several are a tenth cheaper
+  int one = 1;
+  for (int c = 2; c <= most; ++c)
+    if (rest <= kRoom[c] && t[c] < t[one]) one = c;
+  const bool several = best[kMaxParts - 1][rest] * 1.1 < t[one];
+  if (rest == 0 || (!several && one == 1)) {   // whole rounds, or a last one that clusters do not shorten
+    out[0] = {0, batch, 1};
+    return 1;
+  }
+  int parts = 0, b = 0, r = rest;
+  if (full > 0) {
+    out[parts++] = {0, full, 1};
+    b = full;
+  }
+  for (int k = kMaxParts - 1; r > 0; --k) {
+    const int c = several ? pick[k][r] : one, m = r < kRoom[c] ? r : kRoom[c];
+    out[parts++] = {b, m, c};
+    b += m;
+    r -= m;
+  }
+  return parts;
 }
 
 template <int kE, bool kCg>
@@ -644,15 +718,23 @@ extern "C" int lime_lindblad_rk4_f64(const LimeLindbladDesc* d, void* stream) {
   a.n_drive = d->n_drive;
   a.drive_ops = reinterpret_cast<const double2*>(d->drive_ops);
   a.drive_coef = d->drive_coef;
-  const f64::RK4Plan P = f64::plan_rk4(d->n, d->batch, d->k_dense);
-  a.cluster = P.cluster; a.ld = P.ld; a.vcap = P.vcap; a.row_cap = P.row_cap; a.y_smem = P.y_smem;
   // bounded launches: at most ~2^27 complex MACs of GEMM per instance per launch
   const double per_step = 4.0 * (1 + 2 * d->k_dense) * (double)nn * d->n;
   int chunk = (int)fmax(1.0, fmin((double)d->n_steps, 134217728.0 / per_step));
-  for (int s0 = 0; s0 < d->n_steps; s0 += chunk) {
-    a.step0 = s0;
-    a.n_steps = (d->n_steps - s0 < chunk) ? d->n_steps - s0 : chunk;
-    int rc;
+  f64::RK4Part part[f64::kMaxParts];
+  const int parts = f64::split_batch(d->n, d->batch, d->k_dense, d->n_steps, part);
+  for (int i = 0; i < parts; ++i) {
+    const f64::RK4Plan P = f64::plan_rk4(d->n, part[i].cluster, d->k_dense);
+    const int64_t skip = part[i].b0 - a.b0;
+    a.b0 = part[i].b0;
+    a.rho += skip * nn;
+    a.ws += skip * f64::ws_mats(d->k_dense) * nn;
+    a.tr0 += skip;
+    if (a.obs_out) a.obs_out += skip * a.obs_per_inst * a.n_obs;
+    if (a.states) a.states += skip * a.states_per_inst * nn;
+    a.obs_elems -= (size_t)skip * a.obs_per_inst * a.n_obs;
+    a.states_elems -= (size_t)skip * a.states_per_inst * nn;
+    a.cluster = P.cluster; a.ld = P.ld; a.vcap = P.vcap; a.row_cap = P.row_cap; a.y_smem = P.y_smem;
     const auto run = P.cluster > 1 ? (P.e == 1   ? f64::launch_rk4<1, true>
                                       : P.e == 2 ? f64::launch_rk4<2, true>
                                       : P.e == 4 ? f64::launch_rk4<4, true>
@@ -663,8 +745,11 @@ extern "C" int lime_lindblad_rk4_f64(const LimeLindbladDesc* d, void* stream) {
                                       : P.e == 4 ? f64::launch_rk4<4, false>
                                       : P.e == 8 ? f64::launch_rk4<8, false>
                                                  : f64::launch_rk4<0, false>);
-    rc = run(a, P, d->batch, st);
-    if (rc != LIME_OK) return rc;
+    for (int s0 = 0; s0 < d->n_steps; s0 += chunk) {
+      a.step0 = s0;
+      a.n_steps = (d->n_steps - s0 < chunk) ? d->n_steps - s0 : chunk;
+      LIME_TRY(run(a, P, part[i].count, st));
+    }
   }
   return LIME_OK;
 }

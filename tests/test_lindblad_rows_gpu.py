@@ -152,3 +152,29 @@ def test_continues_over_launches():
     gen = engine.LindbladGenerator.build(H, [engine.SiteDephasing(rates)])
     _, _, end = engine.propagate(gen, rho, 0.05, 30, None)
     _close(end, ref[:, -1])
+
+
+@pytest.mark.parametrize('n,B,dense', [(64, 153, 0), (64, 228, 0), (37, 48, 2), (20, 170, 3), (24, 304, 0), (16, 151, 1)])
+def test_batches_in_several_launches(n, B, dense):
+    """A batch split over launches of different cluster sizes: every instance
+    as it comes out alone, observables and states included."""
+    from lime_gb300 import engine
+    g = torch.Generator(device='cuda').manual_seed(n + B)
+
+    def c(*s):
+        return torch.complex(torch.randn(*s, generator=g, device='cuda', dtype=torch.float64),
+                             torch.randn(*s, generator=g, device='cuda', dtype=torch.float64))
+    H = c(B, n, n) / n
+    H = H + H.mH
+    ops = [0.2 * c(B, n, n) / n for _ in range(dense)]
+    rho = c(B, n, n)
+    rho = rho @ rho.mH
+    rho = rho / torch.diagonal(rho, dim1=1, dim2=2).sum(1).real[:, None, None]
+    rho = (rho + rho.mH) / 2
+    args = dict(dt=0.05, n_steps=5, e_ops=engine.Populations(min(n, 7)), states_every=2)
+    o, s, r = engine.propagate(engine.LindbladGenerator.build(H, ops), rho, **args)
+    for b in (0, 1, B // 2, 151 % B, 152 % B, B - 2, B - 1):
+        o1, s1, r1 = engine.propagate(engine.LindbladGenerator.build(H[b], [x[b] for x in ops]), rho[b], **args)
+        # the same products in the same order, whatever the cluster
+        assert (o[b] - o1[0]).abs().max().item() < 1e-14 and (s[b] - s1[0]).abs().max().item() < 1e-14
+        assert (r[b] - r1[0]).abs().max().item() < 1e-14
