@@ -575,10 +575,10 @@ __global__ void init_kernel(Args a, const double2* rho, int batch) {
 // obs[b][slot][o] = Tr(E_o rho_b) = sum_xy E_o[x][y] rho[y][x], fp64 from hi + lo.
 // Only the nonzero entries cost FP64 work (projectors and dipoles are
 // sparse; a zero entry adds exactly zero, and non-finite states are flagged
-// by the stage kernels), so the time is the latency of reading E: a block of
-// 256 threads keeps 8 loads a thread in flight, 128 threads with one each
-// took 108 us for 64 dense 129 x 129 observables.
-constexpr int kObsThreads = 256;
+// by the stage kernels), so the time is the latency of reading E and of the
+// few state elements: 64 dense 129 x 129 observables, 1024 threads with 4
+// loads in flight each, 28 us (256 with 8: 41; 128 with one: 108).
+constexpr int kObsThreads = 1024;
 __device__ __forceinline__ double2 rho_at(const Args& a, size_t base, int x, int y) {
   const size_t er = base + (size_t)x * a.np + y, ei = base + (size_t)(a.np + x) * a.np + y;
   return make_double2(fpconv::widen_f32(a.Phi[er]) + fpconv::widen_f32(a.Plo[er]),
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kObsThreads) observe_kernel(Args a, const doub
   const double2* Eo = E + (e_stride ? (int64_t)(b % a.P) * e_stride : 0) + (int64_t)o * per;
   const size_t base = (size_t)b * inst_floats(a);
   double sr = 0.0, si = 0.0;
-  constexpr int kN = 8;
+  constexpr int kN = 4;
   for (int q0 = threadIdx.x; q0 < per; q0 += kN * kObsThreads) {
     double2 ev[kN];
 #pragma unroll
