@@ -220,6 +220,10 @@ int lime_redfield_build_f64(const LimeRedfieldBuildDesc* d, void* stream);
  *   obs_ops [n_obs][n][n] (eigenbasis); obs_out [n_steps/obs_every][n_rhs][n_obs]
  *           = Tr(E rho_r) after steps obs_every-1, 2*obs_every-1, ...
  *   states  [n_steps/states_every][n^2][n_rhs] or NULL
+ *   workspace lime_redfield_rk4_f64_workspace() bytes.  Up to 8 right-hand
+ *           sides run as one launch for the time loop; with less than that
+ *           but 48 n^2 n_rhs bytes the call runs as a GEMM a stage.  A wait
+ *           inside the loop is bounded; one that expires leaves NaN in rho.
  */
 typedef struct {
   int32_t n, n_rhs, n_steps, n_obs, obs_every, states_every;

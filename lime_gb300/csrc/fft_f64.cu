@@ -292,10 +292,12 @@ extern "C" int lime_fft_f64(const LimeFftDesc* d, void* stream) {
   p.shift = d->shift;
   p.post = reinterpret_cast<const double2*>(d->post);
   const size_t smem = (size_t)m * sizeof(double2);
+  // (one value for every length: calls of other threads set the same attribute)
+  constexpr int kMost = fft::kMaxPow2 * (int)sizeof(double2);
   // a thread takes 8 elements of a pass
   const int nt = m / 8 < 32 ? 32 : m / 8 < fft::kThreads ? m / 8 : fft::kThreads;
   if (l2 >= 0) {
-    LIME_CUDA_TRY(cudaFuncSetAttribute(fft::pow2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LIME_CUDA_TRY(cudaFuncSetAttribute(fft::pow2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
     fft::pow2_kernel<<<d->batch, nt, smem, st>>>(p);
     LIME_CUDA_TRY(cudaGetLastError());
     count_launch();
@@ -303,8 +305,8 @@ extern "C" int lime_fft_f64(const LimeFftDesc* d, void* stream) {
   }
   p.conv = reinterpret_cast<double2*>(d->workspace);      // [batch][m]
   p.chirp = p.conv + (size_t)d->batch * m;                 // [m]: n + m/2 + 1 <= m, n is not a power of two
-  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::chirp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::chirp_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::chirp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  LIME_CUDA_TRY(cudaFuncSetAttribute(fft::chirp_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
   fft::chirp_kernel<<<(n + 63) / 64, 64, 0, st>>>(p);
   LIME_CUDA_TRY(cudaGetLastError());
   fft::chirp_forward_kernel<<<d->batch + 1, nt, smem, st>>>(p);

@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
 template <int kE>
 static int launch_rows(const AdjArgs& a, int batch, int threads, int row_cap, size_t smem, cudaStream_t st) {
   auto kern = adjoint_rows_kernel<kE>;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (one value for every shape: calls of other threads set the same attribute)
+  LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjSmem));
   kern<<<batch, threads, smem, st>>>(a, row_cap, smem);
   LIME_CUDA_TRY(cudaGetLastError());
   count_launch();

@@ -16,9 +16,8 @@
 // batch smaller than the chip is spread over clusters.  Measured per RK4 step
 // against tiled GEMMs of the full Heff and L_k over one CTA: 16-site chain,
 // one instance, 58 -> 4.8 us (a stage's DFMA alone take 0.57 us of its 1.2);
-// 64-site chain, 512 instances, 4.9 -> 0.25 ms; 37 levels with three dense
-// operators, 48 instances, 5.6 -> 0.72 ms; 64 levels, full real H, 600
-// instances, 5.4 -> 2.2 ms.
+// 64-site chain, 512 instances, 4.9 -> 0.24 ms; 37 levels with three dense
+// operators, 48 instances, 5.6 -> 0.61 ms.
 
 #include "rows_f64.cuh"
 
@@ -649,7 +648,8 @@ static int split_batch(int n, int batch, int k_dense, int n_steps, RK4Part* out)
 template <int kE, bool kCg>
 static int launch_rk4(const RK4Args& a, const RK4Plan& P, int batch, cudaStream_t st) {
   auto kern = lindblad_rk4_f64_kernel<kE, kCg>;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+  // (one value for every shape: calls of other threads set the same attribute)
+  LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)((int64_t)batch * P.cluster));
   cfg.blockDim = dim3(P.nt + (kE == 1 ? 32 : 0));

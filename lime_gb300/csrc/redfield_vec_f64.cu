@@ -269,7 +269,8 @@ int begin(const Plan& p, const Run& r, cudaStream_t st) {
 template <int kMode>
 static int launch_mode(const Plan& p, const Args& a, cudaStream_t st) {
   auto kern = rk4_kernel<kMode>;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  // (one value for every shape: calls of other threads set the same attribute)
+  LIME_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)p.ctas);
   cfg.blockDim = dim3(kThreads);

@@ -358,11 +358,8 @@ def split_supported(gen: LindbladGenerator) -> str | None:
 
 
 def m_is_diagonal(gen: LindbladGenerator) -> bool:
-    """Whether M is diagonal (decided once per generator)."""
-    c = gen.split_cache
-    if 'm_diagonal' not in c:
-        c['m_diagonal'] = is_diagonal(gen.m)
-    return c['m_diagonal']
+    """Whether M is diagonal (known from the operators, or a test on the device)."""
+    return bool(gen.split_cache.get('m_diagonal')) or is_diagonal(gen.m)
 
 
 def _pow2_exponent(target: float, bound: float) -> int:
@@ -578,21 +575,18 @@ def _run_stream(gen: LindbladGenerator, rho: torch.Tensor, dt: float, n_steps: i
     n_slots = n_steps // obs_every
     obs_out = torch.zeros((B, max(n_slots, 1), max(n_obs, 1)), dtype=CDT, device=dev)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
-    # one read back: max |rho0|, the operators' largest absolute row sum (once
-    # per generator) and whether device observables are diagonal
-    facts = [torch.view_as_real(rho).abs().max() if rho.numel() else torch.zeros((), dtype=torch.float64, device=dev)]
-    if K and 'lrow' not in gen.split_cache:
-        facts.append(gen.l_dense.abs().sum(-1).max())
+    # one read back: max |rho0|, the operators' largest absolute row sum, and
+    # whether device observables and M are diagonal
     ask_diag = n_obs > 0 and not obs_diag and any(h is None for h in host)
+    ask_m = gen.m is not None and not gen.split_cache.get('m_diagonal')
+    facts = [torch.view_as_real(rho).abs().max() if rho.numel() else torch.zeros((), dtype=torch.float64, device=dev),
+             gen.l_dense.abs().sum(-1).max() if K else None,
+             _off_diagonal(E).double() if ask_diag else None,
+             _off_diagonal(gen.m).double() if ask_m else None]
+    known = iter(torch.stack([f for f in facts if f is not None]).tolist())
+    pmax, lrow, off_e, off_m = [0.0 if f is None else next(known) for f in facts]
     if ask_diag:
-        facts.append(_off_diagonal(E).double())
-    facts = torch.stack(facts).tolist()
-    pmax = facts[0]
-    if K and 'lrow' not in gen.split_cache:
-        gen.split_cache['lrow'] = facts[1]
-    lrow = gen.split_cache['lrow'] if K else 0.0
-    if ask_diag:
-        obs_diag = facts[-1] == 0
+        obs_diag = off_e == 0
     if obs_diag:
         E = torch.diagonal(E, dim1=-2, dim2=-1).contiguous()
     scales = [_pow2_exponent(8192.0 / 1.25, pmax), _pow2_exponent(8192.0 / 1.25, lrow * pmax) if K else 0]
@@ -600,8 +594,8 @@ def _run_stream(gen: LindbladGenerator, rho: torch.Tensor, dt: float, n_steps: i
     l_shared = gen.l_dense is None or gen.l_dense.shape[0] == 1
     # a diagonal M (pure dephasing) goes in as its real diagonal
     m_diag = None
-    if gen.m is not None and m_is_diagonal(gen):
-        m_diag = split_operands_mdiag(gen)
+    if gen.m is not None and off_m == 0:
+        m_diag = torch.diagonal(gen.m, dim1=-2, dim2=-1).real.contiguous()
     G = 1 if (heff_shared and l_shared) else param_batch
     wsb = lib.lime_lindblad_stream_workspace(n, B, G, K)
     ws = torch.empty(wsb + 1024, dtype=torch.uint8, device=dev)
