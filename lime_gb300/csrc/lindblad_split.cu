@@ -56,7 +56,10 @@
 //
 // The epilogue's issue slots are the second bound beside the latency of a
 // stage, so its arithmetic runs on pairs of columns (f32x2.cuh): 4096
-// instances of 64 levels, 20 steps, 4.77 -> 4.48 ms.
+// instances of 64 levels, 20 steps, 4.77 -> 4.48 ms.  The MMAs of a stage are
+// issued by an elected lane from warp-uniform operands (tc::uniform): a stage
+// of the n <= 16 kernel spent 900 clocks on issuing ten of them, now 400, and
+// the same call takes 4.16 ms.
 
 #include "common.cuh"
 #include "f32x2.cuh"
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(kThreads) prepare_a_kernel(const double2* heff
   }
 }
 
-// Issue one MMA pass (thread 0) and commit it to mbar; every thread then
+// Issue one MMA pass (one lane of the calling warp) and commit it to mbar; every thread then
 // waits on mbar itself (bounded), and the next __syncthreads_or turns any
 // thread's timeout into a common abort.  No thread can fall two phases
 // behind: each pass is issued only after a barrier that every thread reaches
@@ -409,21 +412,24 @@ __device__ __forceinline__ void mma_pass(uint32_t tbase, uint64_t desc_b0, uint6
   constexpr uint32_t idesc = tc::idesc_f16(128, 64, 0);
   constexpr uint64_t kDescStep = 2 * kLBO / 16;
   tc::tc_fence_after();
+  if (tc::elect_one()) {
 #pragma unroll
-  for (int ks = 0; ks < 8; ++ks) {
-    const uint64_t d0 = desc_b0 + kDescStep * ks;
-    const uint32_t acc = ks > 0 ? 1u : 0u;
-    if (kExact) {
-      tc::mma_f16_ts(tbase + kColD, tbase + kColA0 + ks * 8, d0, idesc, acc);
-    } else {
-      const uint64_t d1 = desc_b1 + kDescStep * ks;
-      tc::mma_f16_ts(tbase + kColD, tbase + kColA1 + ks * 8, d0, idesc, acc);
-      tc::mma_f16_ts(tbase + kColD, tbase + kColA0 + ks * 8, d1, idesc, 1u);
-      tc::mma_f16_ts(tbase + kColD, tbase + kColA1 + ks * 8, d1, idesc, 1u);
-      tc::mma_f16_ts(tbase + kColD, tbase + kColA2 + ks * 8, d0, idesc, 1u);
+    for (int ks = 0; ks < 8; ++ks) {
+      const uint64_t d0 = desc_b0 + kDescStep * ks;
+      const uint32_t acc = ks > 0 ? 1u : 0u;
+      if (kExact) {
+        tc::mma_f16_ts(tbase + kColD, tbase + kColA0 + ks * 8, d0, idesc, acc);
+      } else {
+        const uint64_t d1 = desc_b1 + kDescStep * ks;
+        tc::mma_f16_ts(tbase + kColD, tbase + kColA1 + ks * 8, d0, idesc, acc);
+        tc::mma_f16_ts(tbase + kColD, tbase + kColA0 + ks * 8, d1, idesc, 1u);
+        tc::mma_f16_ts(tbase + kColD, tbase + kColA1 + ks * 8, d1, idesc, 1u);
+        tc::mma_f16_ts(tbase + kColD, tbase + kColA2 + ks * 8, d0, idesc, 1u);
+      }
     }
+    tc::mma_commit(mbar);
   }
-  tc::mma_commit(mbar);
+  __syncwarp();
 }
 
 template <bool kDrive>
@@ -451,10 +457,11 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tbase = S.tmem_base;
+  const uint32_t tbase = tc::uniform(S.tmem_base);
+  const bool mma_warp = tc::uniform((uint32_t)t >> 5) == 0;   // one of its lanes issues the MMAs
   const uint32_t lane_addr = tbase + ((uint32_t)(lq * 32) << 16);
-  const uint64_t desc_b0 = tc::smem_desc_noswizzle(tc::smem_u32(S.bop[0]), kLBO, kSBO);
-  const uint64_t desc_b1 = tc::smem_desc_noswizzle(tc::smem_u32(S.bop[1]), kLBO, kSBO);
+  const uint64_t desc_b0 = tc::uniform64(tc::smem_desc_noswizzle(tc::smem_u32(S.bop[0]), kLBO, kSBO));
+  const uint64_t desc_b1 = tc::uniform64(tc::smem_desc_noswizzle(tc::smem_u32(S.bop[1]), kLBO, kSBO));
   const uint32_t brow = (uint32_t)(i >> 3) * kSBO + (uint32_t)(i & 7) * 16u;
   const uint32_t bchunk0 = (is_re ? 0u : 8u) + 4u * (uint32_t)h;
   const float tsign = is_re ? 1.f : -1.f;      // u = own +- transposed element
@@ -697,7 +704,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
         tc::fence_proxy_async_smem();
         tc::tc_fence_before();
         __syncthreads();
-        if (t == 0) mma_pass<false>(tbase, desc_b0, desc_b1, &S.mbar);
+        if (mma_warp) mma_pass<false>(tbase, desc_b0, desc_b1, &S.mbar);
         if (tr_pending) {
           if (t == 0 && fabs(S.trp[0] + S.trp[1] - S.tr0) > a.trace_tol * fmax(1.0, fabs(S.tr0)))
             flags |= LIME_FLAG_TRACE_DRIFT;
@@ -714,7 +721,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
           aborted = true;
           break;
         }
-        if (t == 0) mma_pass<true>(tbase, desc_b0, desc_b1, &S.mbar);
+        if (mma_warp) mma_pass<true>(tbase, desc_b0, desc_b1, &S.mbar);
         timed_out = tc::mbar_wait_bounded(&S.mbar, phase, a.max_wait) ? 0 : 1;
         phase ^= 1u;
         tc::tc_fence_after();
@@ -924,8 +931,8 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
 //
 // Bound: a stage's chain of MMA, TMEM load, transpose and B store (one
 // instance), the issue slots of the epilogue (batches).  Measured against the
-// 64-wide kernel: 4096 instances, 20 steps, n = 16: 4.66 -> 0.69 ms, n = 32:
-// 4.70 -> 1.36 ms; one 16-site chain 3.1 -> 1.0 us a stage.
+// 64-wide kernel: 4096 instances, 20 steps, n = 16: 4.66 -> 0.68 ms, n = 32:
+// 4.70 -> 1.15 ms; one 16-site chain 3.1 -> 0.8 us a stage.
 template <int kW>
 struct __align__(128) SmallSmem {
   uint8_t bop[2][4 * kW * kW];           // B0, B1: kW (N) x 2 kW (K) fp16
@@ -966,22 +973,28 @@ __device__ __forceinline__ void tmem_ld(uint32_t addr, float (&v)[kC]) {
   for (int c = 0; c < kC; ++c) v[c] = __uint_as_float(r[c / 8][c % 8]);
 }
 
-template <int kW, bool kDual>
-__device__ __forceinline__ void small_mma(uint32_t tbase, uint64_t desc_b0, uint64_t desc_b1, bool small, bool exact) {
+// the small products and / or the exact one of a stage, by one lane of the calling warp
+template <int kW, bool kDual, bool kSmall, bool kExact>
+__device__ __forceinline__ void small_mma(uint32_t tbase, uint64_t desc_b0, uint64_t desc_b1, uint64_t* mbar) {
   using Sh = SmallShape<kW, kDual>;
   constexpr uint32_t idesc = tc::idesc_f16(128, kW, 0);
+  tc::tc_fence_after();
+  if (tc::elect_one()) {
 #pragma unroll
-  for (int ks = 0; ks < kW / 8; ++ks) {
-    const uint64_t d0 = desc_b0 + (uint64_t)(2 * kLBO / 16) * ks, d1 = desc_b1 + (uint64_t)(2 * kLBO / 16) * ks;
-    const uint32_t acc = ks > 0 ? 1u : 0u, a = tbase + 8 * ks;
-    if (small) {
-      tc::mma_f16_ts(tbase + Sh::kD1, a + kW, d0, idesc, acc);
-      tc::mma_f16_ts(tbase + Sh::kD1, a, d1, idesc, 1u);
-      tc::mma_f16_ts(tbase + Sh::kD1, a + kW, d1, idesc, 1u);
-      tc::mma_f16_ts(tbase + Sh::kD1, a + 2 * kW, d0, idesc, 1u);
+    for (int ks = 0; ks < kW / 8; ++ks) {
+      const uint64_t d0 = desc_b0 + (uint64_t)(2 * kLBO / 16) * ks, d1 = desc_b1 + (uint64_t)(2 * kLBO / 16) * ks;
+      const uint32_t acc = ks > 0 ? 1u : 0u, a = tbase + 8 * ks;
+      if (kSmall) {
+        tc::mma_f16_ts(tbase + Sh::kD1, a + kW, d0, idesc, acc);
+        tc::mma_f16_ts(tbase + Sh::kD1, a, d1, idesc, 1u);
+        tc::mma_f16_ts(tbase + Sh::kD1, a + kW, d1, idesc, 1u);
+        tc::mma_f16_ts(tbase + Sh::kD1, a + 2 * kW, d0, idesc, 1u);
+      }
+      if (kExact) tc::mma_f16_ts(tbase + Sh::kD, a, d0, idesc, acc);
     }
-    if (exact) tc::mma_f16_ts(tbase + Sh::kD, a, d0, idesc, acc);
+    tc::mma_commit(mbar);
   }
+  __syncwarp();
 }
 
 template <int kW, bool kDual>
@@ -1010,10 +1023,11 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tbase = S.tmem_base;
+  const uint32_t tbase = tc::uniform(S.tmem_base);
+  const bool mma_warp = tc::uniform((uint32_t)t >> 5) == 0;
   const uint32_t lane_addr = tbase + ((uint32_t)(q * 32) << 16);
-  const uint64_t desc_b0 = tc::smem_desc_noswizzle(tc::smem_u32(S.bop[0]), kLBO, kS);
-  const uint64_t desc_b1 = tc::smem_desc_noswizzle(tc::smem_u32(S.bop[1]), kLBO, kS);
+  const uint64_t desc_b0 = tc::uniform64(tc::smem_desc_noswizzle(tc::smem_u32(S.bop[0]), kLBO, kS));
+  const uint64_t desc_b1 = tc::uniform64(tc::smem_desc_noswizzle(tc::smem_u32(S.bop[1]), kLBO, kS));
   const uint32_t bseg = (uint32_t)(i >> 3) * kS + (uint32_t)(i & 7) * 16u +
                         ((is_re ? 0u : (uint32_t)kW / 8) + (uint32_t)(kC / 8 * h)) * kLBO;
   const float tsign = is_re ? 1.f : -1.f;
@@ -1181,11 +1195,7 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
         tc::fence_proxy_async_smem();
         tc::tc_fence_before();
         __syncthreads();
-        if (t == 0) {
-          tc::tc_fence_after();
-          small_mma<kW, kDual>(tbase, desc_b0, desc_b1, true, kDual);
-          tc::mma_commit(&S.mbar);
-        }
+        if (mma_warp) small_mma<kW, kDual, true, kDual>(tbase, desc_b0, desc_b1, &S.mbar);
         if (tr_pending) trace_check();
         const float magic = row_magic(row_bound());
         int timed_out = tc::mbar_wait_bounded(&S.mbar, phase, a.max_wait) ? 0 : 1;
@@ -1212,11 +1222,7 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
             aborted = true;
             break;
           }
-          if (t == 0) {
-            tc::tc_fence_after();
-            small_mma<kW, kDual>(tbase, desc_b0, desc_b1, false, true);
-            tc::mma_commit(&S.mbar);
-          }
+          if (mma_warp) small_mma<kW, kDual, false, true>(tbase, desc_b0, desc_b1, &S.mbar);
           timed_out = tc::mbar_wait_bounded(&S.mbar, phase, a.max_wait) ? 0 : 1;
           phase ^= 1u;
           tc::tc_fence_after();
@@ -1606,10 +1612,10 @@ extern "C" int lime_lindblad_rk4_split(const LimeLindbladSplitDesc* d, void* str
   }
   // Dimensions up to 32 without a drive leave the 64-wide kernel, whose time
   // does not depend on n (20 steps of 16 instances 0.35 ms, of 4096 4.7 ms; at
-  // n = 16 0.17 and 0.69, at n = 32 0.21 and 1.36 ms).  One wait a stage
+  // n = 16 0.16 and 0.68, at n = 32 0.18 and 1.15 ms).  One wait a stage
   // (kDual) while its CTAs hold the batch in one round; beyond that the other
-  // form holds twice as many (n = 32, 608 instances in one round: 0.27 ms,
-  // where 304 in one round of the first take 0.22).
+  // form holds twice as many (n = 32, 608 instances in one round: 0.25 ms,
+  // where 304 in one round of the first take 0.19).
   void (*kern)(split::Args) = driven ? split::lindblad_rk4_split_kernel<true> : split::lindblad_rk4_split_kernel<false>;
   size_t smem = sizeof(split::Smem) + 1024;
   int threads = split::kThreads, resident = 2;

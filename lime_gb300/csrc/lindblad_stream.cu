@@ -329,27 +329,30 @@ __global__ void __launch_bounds__(sg::kThreads, 1) gemm_groups_kernel(const __gr
   sg::setup(S);
   chain_wait();
   sg::Seq q;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int t = threadIdx.x, warp = (int)tc::uniform((uint32_t)t >> 5), lane = t & 31;
   auto group_of = [&](int item) {
     int gi = 0;
     while (gi + 1 < m.n_groups && item >= m.start[gi + 1]) ++gi;
     return gi;
   };
-  if (warp < 2) {
-    if (lane == 0) {
-      bool alive = true;
-      for (int item = blockIdx.x; item < m.n_items && alive; item += gridDim.x) {
-        const int gi = group_of(item);
-        sg::Tile T;
-        int b, mt, nt;
-        gemm_tile_of<kZ>(m.g[gi], item - m.start[gi], T, b, mt, nt);
-        alive = warp == 0 ? sg::seq_produce(S, T, q) : sg::seq_mma(S, T, q);
-      }
-      if (warp == 0)
-        sg::seq_produce_end(S, q, m.g[0].max_wait);
-      else
-        sg::seq_mma_end(S, m.g[0].max_wait);
+  auto tiles = [&](const auto& role) {
+    bool alive = true;
+    for (int item = blockIdx.x; item < m.n_items && alive; item += gridDim.x) {
+      const int gi = group_of(item);
+      sg::Tile T;
+      int b, mt, nt;
+      gemm_tile_of<kZ>(m.g[gi], item - m.start[gi], T, b, mt, nt);
+      alive = role(T);
     }
+  };
+  if (warp == 0) {
+    if (lane == 0) {
+      tiles([&](const sg::Tile& T) { return sg::seq_produce(S, T, q); });
+      sg::seq_produce_end(S, q, m.g[0].max_wait);
+    }
+  } else if (warp == 1) {
+    tiles([&](const sg::Tile& T) { return sg::seq_mma(S, T, q); });
+    sg::seq_mma_end(S, m.g[0].max_wait);
   } else {
     const float* ft = S.lo;
     for (int item = blockIdx.x; item < m.n_items; item += gridDim.x) {

@@ -296,13 +296,36 @@ __device__ __forceinline__ void teardown(Smem& S, int32_t* status) {
   }
 }
 
+// The MMAs of one chunk in ring stage `stage` into D0 at d0 and D1 128 columns
+// further (first: they overwrite), committed to `empty` and, if given, `accf`;
+// by one lane of the calling warp.
+__device__ __forceinline__ void issue_chunk(const void* stage, uint32_t d0, bool first, uint64_t* empty,
+                                            uint64_t* accf) {
+  constexpr uint32_t idesc = tc::idesc_f16(kBM, kBN, 0);
+  const uint32_t base = tc::uniform(operand_base(stage)), d1 = d0 + 128u;
+  if (tc::elect_one()) {
+#pragma unroll
+    for (int ks = 0; ks < kCK / 16; ++ks) {
+      const uint32_t acc = (first && ks == 0) ? 0u : 1u;
+      tc::mma_f16_ss(d0, operand(base, 0, ks), operand(base, 3, ks), idesc, acc);
+      tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 3, ks), idesc, acc);
+      tc::mma_f16_ss(d1, operand(base, 0, ks), operand(base, 4, ks), idesc, 1u);
+      tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 4, ks), idesc, 1u);
+      tc::mma_f16_ss(d1, operand(base, 2, ks), operand(base, 3, ks), idesc, 1u);
+    }
+    tc::mma_commit(empty);
+    if (accf != nullptr) tc::mma_commit(accf);
+  }
+  __syncwarp();
+}
+
 // The tile's main loop.  Returns true on the kEpiThreads epilogue threads, which on
 // return have parked C[r][c] * row_inv[r] * inv_sb at S.tile()[c * kFStride
 // + r] and passed a named barrier together (unless S.abort is set: a wait
 // expired and the tile is not valid); false on the producer and MMA warps.
 __device__ __forceinline__ bool mainloop(Smem& S, const Tile& T) {
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const uint32_t tbase = S.tmem_base;
+  const int t = threadIdx.x, warp = (int)tc::uniform((uint32_t)t >> 5), lane = t & 31;
+  const uint32_t tbase = tc::uniform(S.tmem_base);
   const int KC = T.n_chunks;
 
   if (warp == 0) {
@@ -335,41 +358,24 @@ __device__ __forceinline__ bool mainloop(Smem& S, const Tile& T) {
     return false;
   }
   if (warp == 1) {
-    // ---------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc::idesc_f16(kBM, kBN, 0);
-      for (int c = 0; c < KC; ++c) {
-        const int s = c % kStages;
-        const uint32_t ph = (uint32_t)(c / kStages) & 1u;
-        const int p = c / kGroup, b = p & 1;
-        const bool first = (c % kGroup) == 0;
-        const bool last = (c % kGroup) == kGroup - 1;
-        if (!tc::mbar_wait_bounded(&S.full[s], ph, T.max_wait)) { atomicExch(&S.abort, 1); break; }
-        if (first && !tc::mbar_wait_bounded(&S.acce[b], ((uint32_t)(p >> 1) & 1u) ^ 1u, T.max_wait)) {
-          atomicExch(&S.abort, 1);
-          break;
-        }
-        if (*(volatile int*)&S.abort) break;
-        tc::tc_fence_after();
-        const uint32_t d0 = tbase + (uint32_t)(2 * b) * 128u;
-        const uint32_t d1 = d0 + 128u;
-        const uint32_t base = operand_base(S.stage[s][0]);
-#pragma unroll
-        for (int ks = 0; ks < kCK / 16; ++ks) {
-          const uint32_t acc = (first && ks == 0) ? 0u : 1u;
-          tc::mma_f16_ss(d0, operand(base, 0, ks), operand(base, 3, ks), idesc, acc);
-          tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 3, ks), idesc, acc);
-          tc::mma_f16_ss(d1, operand(base, 0, ks), operand(base, 4, ks), idesc, 1u);
-          tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 4, ks), idesc, 1u);
-          tc::mma_f16_ss(d1, operand(base, 2, ks), operand(base, 3, ks), idesc, 1u);
-        }
-        tc::mma_commit(&S.empty[s]);
-        if (last) tc::mma_commit(&S.accf[b]);
-      }
-      // every MMA this thread issued has completed before TMEM is released
-      tc::mma_commit(&S.drain);
-      tc::mbar_wait_bounded(&S.drain, 0u, T.max_wait);
+    // ---------------- MMA issuer: the warp waits together, one lane issues
+    for (int c = 0; c < KC; ++c) {
+      const int s = c % kStages;
+      const uint32_t ph = (uint32_t)(c / kStages) & 1u;
+      const int p = c / kGroup, b = p & 1;
+      const bool first = (c % kGroup) == 0;
+      const bool last = (c % kGroup) == kGroup - 1;
+      bool ok = tc::mbar_wait_bounded(&S.full[s], ph, T.max_wait);
+      if (first) ok = ok && tc::mbar_wait_bounded(&S.acce[b], ((uint32_t)(p >> 1) & 1u) ^ 1u, T.max_wait);
+      if (!ok) atomicExch(&S.abort, 1);
+      if (__any_sync(0xffffffffu, !ok || *(volatile int*)&S.abort)) break;
+      tc::tc_fence_after();
+      issue_chunk(S.stage[s][0], tbase + (uint32_t)(2 * b) * 128u, first, &S.empty[s], last ? &S.accf[b] : nullptr);
     }
+    // every MMA this warp issued has completed before TMEM is released
+    if (tc::elect_one()) tc::mma_commit(&S.drain);
+    __syncwarp();
+    tc::mbar_wait_bounded(&S.drain, 0u, T.max_wait);
     return false;
   }
 
@@ -496,48 +502,31 @@ __device__ __forceinline__ void seq_produce_end(Smem& S, const Seq& q, uint32_t 
     tc::mbar_wait_bounded(&S.full[c % kStages], (uint32_t)(c / kStages) & 1u, max_wait);
 }
 
-// MMA issuer (warp 1, lane 0): the tile's MMAs, one accumulator group per
+// MMA issuer (warp 1, all lanes): the tile's MMAs, one accumulator group per
 // 128 K into D0/D1 buffer gp & 1.
 __device__ __forceinline__ bool seq_mma(Smem& S, const Tile& T, Seq& q) {
-  constexpr uint32_t idesc = tc::idesc_f16(kBM, kBN, 0);
-  const uint32_t tbase = S.tmem_base;
+  const uint32_t tbase = tc::uniform(S.tmem_base);
   for (int c = 0; c < T.n_chunks; ++c, ++q.gc) {
     const int s = q.gc % kStages;
     const uint32_t ph = (uint32_t)(q.gc / kStages) & 1u;
     const int b = q.gp & 1;
     const bool first = (c % kGroup) == 0;
     const bool last = (c % kGroup) == kGroup - 1;
-    if (!seq_wait(S, &S.full[s], ph, T.max_wait)) { atomicExch(&S.abort, 1); return false; }
-    if (first && !seq_wait(S, &S.acce[b], ((uint32_t)(q.gp >> 1) & 1u) ^ 1u, T.max_wait)) {
-      atomicExch(&S.abort, 1);
-      return false;
-    }
-    if (*(volatile int*)&S.abort) return false;
+    bool ok = seq_wait(S, &S.full[s], ph, T.max_wait);
+    if (first) ok = ok && seq_wait(S, &S.acce[b], ((uint32_t)(q.gp >> 1) & 1u) ^ 1u, T.max_wait);
+    if (!ok) atomicExch(&S.abort, 1);
+    if (__any_sync(0xffffffffu, !ok || *(volatile int*)&S.abort)) return false;
     tc::tc_fence_after();
-    const uint32_t d0 = tbase + (uint32_t)(2 * b) * 128u;
-    const uint32_t d1 = d0 + 128u;
-    const uint32_t base = operand_base(S.stage[s][0]);
-#pragma unroll
-    for (int ks = 0; ks < kCK / 16; ++ks) {
-      const uint32_t acc = (first && ks == 0) ? 0u : 1u;
-      tc::mma_f16_ss(d0, operand(base, 0, ks), operand(base, 3, ks), idesc, acc);
-      tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 3, ks), idesc, acc);
-      tc::mma_f16_ss(d1, operand(base, 0, ks), operand(base, 4, ks), idesc, 1u);
-      tc::mma_f16_ss(d1, operand(base, 1, ks), operand(base, 4, ks), idesc, 1u);
-      tc::mma_f16_ss(d1, operand(base, 2, ks), operand(base, 3, ks), idesc, 1u);
-    }
-    tc::mma_commit(&S.empty[s]);
-    if (last) {
-      tc::mma_commit(&S.accf[b]);
-      ++q.gp;
-    }
+    issue_chunk(S.stage[s][0], tbase + (uint32_t)(2 * b) * 128u, first, &S.empty[s], last ? &S.accf[b] : nullptr);
+    if (last) ++q.gp;
   }
   return true;
 }
 
 // MMA issuer, after its last tile: every MMA has completed before TMEM is released
 __device__ __forceinline__ void seq_mma_end(Smem& S, uint32_t max_wait) {
-  tc::mma_commit(&S.drain);
+  if (tc::elect_one()) tc::mma_commit(&S.drain);
+  __syncwarp();
   tc::mbar_wait_bounded(&S.drain, 0u, max_wait);
 }
 

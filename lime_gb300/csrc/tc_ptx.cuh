@@ -92,6 +92,25 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// ---------------------------------------------------------------- one thread of a warp
+// The tensor-core instructions take their operands from warp-uniform
+// registers.  A value that the compiler knows to be uniform (uniform(x)) in a
+// branch that it knows to be uniform, with one lane elected in it, goes there
+// once; computed by "if (threadIdx.x == 0)" it is moved for every instruction.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ uint64_t uniform64(uint64_t x) {
+  return (uint64_t)uniform((uint32_t)(x >> 32)) << 32 | uniform((uint32_t)x);
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r));
+  return r != 0;
+}
+
 // ---------------------------------------------------------------- MMA
 // D[tmem] (+)= A[tmem] * B[smem desc], kind::f16 (fp16/bf16 operands, fp32 accumulate).
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
