@@ -93,9 +93,9 @@ struct __align__(1024) Smem {
   float smax[2][kThreads];               // per-thread max |B| of the last written stage input
   double red[2][kThreads / 32];
   float redf[kThreads / 32];
-  double trp[2];                         // trace partial sums of the two warps owning the diagonal
+  double diag[kN];                       // diagonal after the last step, for the trace check
   double trs[2];                         // partial traces of rho(0) (the same two warps)
-  double tr0;                            // trace of the instance's rho(0)
+  double tr0, tr_lim;                    // trace of the instance's rho(0), bound on its drift
   int eb;                                // the instance's B scale exponent b
   uint64_t mbar;
   uint32_t tmem_base;
@@ -637,6 +637,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
     S.smax[g & 1][t] = mx;
     if (t == 0) {   // read after the barriers below (kept out of the step loop's registers)
       S.tr0 = S.trs[0] + S.trs[1];
+      S.tr_lim = a.trace_tol * fmax(1.0, fabs(S.tr0));
       S.eb = eb;
     }
     __syncthreads();   // publishes smax
@@ -648,7 +649,19 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
 #pragma unroll
       for (int c = 0; c < 4; ++c) store_b8(S, brow + (bchunk0 + c) * kLBO, rho + 4 * c, magic, dummy);
     }
-    bool tr_pending = false;   // a trace recorded after the last step awaits its check
+    bool tr_pending = false;   // the diagonal after the last step awaits its trace check
+    // by warp 1, off the path of the warps that own the diagonal: five double
+    // additions in a row are as long as the rest of the readout (4096 instances,
+    // 20 steps, 4.16 -> 4.08 ms)
+    auto trace_check = [&]() {
+      if (warp == 1) {
+        double v = S.diag[t & 31] + S.diag[32 + (t & 31)];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((t & 31) == 0 && fabs(v - S.tr0) > S.tr_lim) flags |= LIME_FLAG_TRACE_DRIFT;
+      }
+      tr_pending = false;
+    };
 
 #pragma unroll 1
     for (int step = 0; step < a.n_steps; ++step) {
@@ -705,11 +718,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
         tc::tc_fence_before();
         __syncthreads();
         if (mma_warp) mma_pass<false>(tbase, desc_b0, desc_b1, &S.mbar);
-        if (tr_pending) {
-          if (t == 0 && fabs(S.trp[0] + S.trp[1] - S.tr0) > a.trace_tol * fmax(1.0, fabs(S.tr0)))
-            flags |= LIME_FLAG_TRACE_DRIFT;
-          tr_pending = false;
-        }
+        if (tr_pending) trace_check();   // while the MMAs run
         int timed_out = tc::mbar_wait_bounded(&S.mbar, phase, a.max_wait) ? 0 : 1;
         phase ^= 1u;
         tc::tc_fence_after();
@@ -855,14 +864,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
           }
         }
         if (a.trace_tol > 0.0) {
-          // the diagonal lives in warps 2 (i < 32) and 7 (i >= 32); their sums
-          // are compared with tr0 by thread 0 after the next barrier
-          if (warp == 2 || warp == 7) {
-            double v = (diag_owner && i < n) ? dval : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((t & 31) == 0) S.trp[warp == 7 ? 1 : 0] = v;
-          }
+          if (diag_owner) S.diag[i] = i < n ? dval : 0.0;
           tr_pending = true;
         }
       }
@@ -896,8 +898,7 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
       }
     }
     __syncthreads();   // smax / rlo of this instance are no longer read
-    if (tr_pending && t == 0 && fabs(S.trp[0] + S.trp[1] - S.tr0) > a.trace_tol * fmax(1.0, fabs(S.tr0)))
-      flags |= LIME_FLAG_TRACE_DRIFT;
+    if (tr_pending) trace_check();
   }
 
   if (aborted) {
@@ -942,7 +943,7 @@ struct __align__(128) SmallSmem {
   float obsp[2][128];                    // dense observables: partial sums of the first column half
   double red[2][4];
   float redf[4];
-  double trp[2], trs[2], tr0;
+  double diag[kW], trs[2], tr0, tr_lim;  // diag: of the last step, or its two halves' sums
   int eb;
   uint64_t mbar;
   uint32_t tmem_base;
@@ -1168,6 +1169,7 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
     S.smax[g & 1][t] = mx;
     if (t == 0) {
       S.tr0 = S.trs[0] + S.trs[1];
+      S.tr_lim = a.trace_tol * fmax(1.0, fabs(S.tr0));
       S.eb = eb;
     }
     __syncthreads();
@@ -1182,9 +1184,21 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
       for (int c = 0; c < kC / 8; ++c) store_b8(S, bseg + c * kLBO, rho + 4 * c, magic, dummy);
     }
     bool tr_pending = false;
+    // the diagonal's sum by warp 1 while the next MMAs run (kW = 32: one chain
+    // of 500 steps 2.98 -> 2.86 ms), or by the warps that own it (kW = 16, whose
+    // MMAs are too short to hide it: 4096 instances 0.69 and 0.67 ms)
+    constexpr bool kAside = kW == 32;
     auto trace_check = [&]() {
-      if (t == 0 && fabs(S.trp[0] + S.trp[1] - S.tr0) > a.trace_tol * fmax(1.0, fabs(S.tr0)))
+      if (kAside) {
+        if (q == 1) {
+          double v = S.diag[i % kW];
+#pragma unroll
+          for (int o = kW / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (i == 0 && fabs(v - S.tr0) > S.tr_lim) flags |= LIME_FLAG_TRACE_DRIFT;
+        }
+      } else if (t == 0 && fabs(S.diag[0] + S.diag[1] - S.tr0) > S.tr_lim) {
         flags |= LIME_FLAG_TRACE_DRIFT;
+      }
       tr_pending = false;
     };
 
@@ -1349,11 +1363,13 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
           }
         }
         if (a.trace_tol > 0.0) {
-          if (is_re) {
+          if (kAside) {
+            if (diag_owner) S.diag[i] = i < n ? dval : 0.0;
+          } else if (is_re) {
             double v = (diag_owner && i < n) ? dval : 0.0;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (i == 0) S.trp[h] = v;
+            if (i == 0) S.diag[h] = v;
           }
           tr_pending = true;
         }
