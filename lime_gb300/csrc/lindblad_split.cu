@@ -59,7 +59,7 @@
 // instances of 64 levels, 20 steps, 4.77 -> 4.48 ms.  The MMAs of a stage are
 // issued by an elected lane from warp-uniform operands (tc::uniform): a stage
 // of the n <= 16 kernel spent 900 clocks on issuing ten of them, now 400, and
-// the same call takes 4.16 ms.
+// the same call takes 4.08 ms.
 
 #include "common.cuh"
 #include "f32x2.cuh"
