@@ -9,6 +9,7 @@ namespace f64 {
 struct AdjArgs {
   int n, param_batch, seg_steps, step0, total_steps, k_dense, n_obs, obs_diag, obs_every, obs_per_inst;
   double dt;
+  Sixth sixth;
   const double2* ckpt;
   double2* lam;
   const double2* heff; int64_t heff_stride;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "../../include/lime_gb300.h"
 
@@ -88,6 +89,28 @@ __device__ __forceinline__ float rk4_final_f32(float x, float acc, float f, floa
   const float hi2 = __fadd_rn(sum, l);
   lo = __fsub_rn(l, __fsub_rn(hi2, sum));
   return hi2;
+}
+
+// dt / 6 as a 24-bit number and the rest.  One rounded factor would stretch
+// every step's increment by the same relative error, which grows with the
+// number of steps where independent roundings grow with its root: 1500
+// oscillators, 4000 steps, rms error 1.2e-14 against 2.0e-15.
+struct Sixth {
+  double hi, lo;
+};
+inline Sixth sixth_of(double dt) {
+  const double s = dt / 6.0;
+  uint64_t u;
+  memcpy(&u, &s, 8);
+  u &= ~((1ull << 29) - 1);
+  Sixth c;
+  memcpy(&c.hi, &u, 8);
+  c.lo = (dt - 6.0 * c.hi) / 6.0;   // the difference is exact
+  return c;
+}
+// x + dt / 6 * sum, the product rounded once
+__device__ __forceinline__ double rk4_final_f64(double x, double sum, Sixth c) {
+  return x + fma(c.hi, sum, c.lo * sum);
 }
 
 // ---------------------------------------------------------------- launches in a chain

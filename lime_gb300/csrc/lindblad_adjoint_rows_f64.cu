@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
     __syncthreads();
     items([&](Idx e, const Item& it, int u) {
       const double f = rhs(F, cF, m, y4, it, u);
-      const double v = fma(dt6, sum[e] + f, own(r, it));
+      const double v = rk4_final_f64(own(r, it), sum[e] + f, a.sixth);
       put(nxt, it, v);
       if (xs) put(xs, it, v);
     });

@@ -397,7 +397,7 @@ extern "C" int lime_lindblad_adjoint_f64(const LimeAdjointDesc* d, void* stream)
   a.total_steps = d->total_steps; a.k_dense = d->k_dense; a.n_obs = d->n_obs; a.obs_diag = d->obs_diag;
   a.obs_every = d->obs_every > 0 ? d->obs_every : 1;
   a.obs_per_inst = d->total_steps / a.obs_every;
-  a.dt = d->dt;
+  a.dt = d->dt; a.sixth = sixth_of(d->dt);
   a.ckpt = reinterpret_cast<const double2*>(d->ckpt);
   a.lam = reinterpret_cast<double2*>(d->lam);
   a.heff = reinterpret_cast<const double2*>(d->heff); a.heff_stride = d->heff_stride;

@@ -42,6 +42,7 @@ __host__ __device__ inline int64_t ws_mats(int k_dense) { return k_dense > 0 ? 6
 struct RK4Args {
   int n, param_batch, n_steps, k_dense, n_obs, obs_diag, states_every, states_per_inst, step0;
   double dt, trace_tol;
+  Sixth sixth;
   double2* rho;
   const double2* heff;    int64_t heff_stride;
   const double2* m;       int64_t m_stride;
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(kE == 1 ? kMaxThreads + 32 : kMaxThreads, 1) l
   };
   stage_sync();
 
-  const double dt = a.dt, dt2 = a.dt / 2.0, dt6 = a.dt / 6.0;
+  const double dt = a.dt, dt2 = a.dt / 2.0;
   int flags = 0, cur = 0;
   // trace of the state after the last step: the helper sums its lanes' parts
   // and compares while the workers are a stage further
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kE == 1 ? kMaxThreads + 32 : kMaxThreads, 1) l
           ac = fma(2.0, f, ac);
           return fma(s == 2 ? dt : dt2, f, r);
         }
-        r = fma(dt6, ac + f, r);
+        r = rk4_final_f64(r, ac + f, a.sixth);
         if (!isfinite(r)) flags |= LIME_FLAG_NONFINITE;
         return r;
       };
@@ -699,7 +700,7 @@ extern "C" int lime_lindblad_rk4_f64(const LimeLindbladDesc* d, void* stream) {
   a.n = d->n; a.param_batch = pb; a.k_dense = d->k_dense; a.n_obs = d->n_obs; a.obs_diag = d->obs_diag;
   a.states_every = d->states ? d->states_every : 1;
   a.states_per_inst = d->states ? d->n_steps / d->states_every : 0;
-  a.dt = d->dt; a.trace_tol = d->trace_tol;
+  a.dt = d->dt; a.sixth = sixth_of(d->dt); a.trace_tol = d->trace_tol;
   a.rho = reinterpret_cast<double2*>(d->rho);
   a.heff = reinterpret_cast<const double2*>(d->heff); a.heff_stride = d->heff_stride;
   a.m = reinterpret_cast<const double2*>(d->m); a.m_stride = d->m_stride;

@@ -34,6 +34,7 @@ struct Args {
   int D, R, F, outs, team, red, l_smem, cluster;
   int step0, n_steps, states_every, obs_every;
   double dt;
+  Sixth sixth;
   const double2* L;
   double2* P;
   ulonglong2* xch;       // [2][F]
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(kThreads, 1) rk4_kernel(Args a) {
   if (kMode == kCluster) cluster_sync();   // peers are running before the first remote store
   __syncthreads();
 
-  const double dt = a.dt, dt2 = a.dt / 2.0, dt6 = a.dt / 6.0;
+  const double dt = a.dt, dt2 = a.dt / 2.0;
   unsigned long long tag = (unsigned long long)a.step0 * 4u;   // of the input of the current stage
   int cur = 0;
   for (int step = 0; step < a.n_steps; ++step) {
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1) rk4_kernel(Args a) {
             ac = fma(2.0, f, ac);
             nx = fma(s == 2 ? dt : dt2, f, p);
           } else {
-            nx = fma(dt6, ac + f, p);
+            nx = rk4_final_f64(p, ac + f, a.sixth);
           }
         }
         __syncwarp();
@@ -300,7 +301,7 @@ int launch(const Plan& p, const Run& r, int step0, int steps, double2* hist, cud
   a.step0 = step0; a.n_steps = steps;
   a.states = r.states; a.states_every = r.states_every > 0 ? r.states_every : 1;
   a.hist = hist; a.obs_every = r.obs_every > 0 ? r.obs_every : 1;
-  a.dt = r.dt; a.L = r.L; a.P = r.P;
+  a.dt = r.dt; a.sixth = sixth_of(r.dt); a.L = r.L; a.P = r.P;
   a.xch = reinterpret_cast<ulonglong2*>(r.ws);
   return p.mode == kSolo ? launch_mode<kSolo>(p, a, st)
                          : p.mode == kCluster ? launch_mode<kCluster>(p, a, st) : launch_mode<kGrid>(p, a, st);
