@@ -222,8 +222,12 @@ int lime_redfield_build_f64(const LimeRedfieldBuildDesc* d, void* stream);
  *   states  [n_steps/states_every][n^2][n_rhs] or NULL
  *   workspace lime_redfield_rk4_f64_workspace() bytes.  Up to 8 right-hand
  *           sides run as one launch for the time loop; with less than that
- *           but 48 n^2 n_rhs bytes the call runs as a GEMM a stage.  A wait
- *           inside the loop is bounded; one that expires leaves NaN in rho.
+ *           but 48 n^2 n_rhs bytes the call runs as a GEMM a stage.
+ * From some sizes on the SMs exchange the stages of that launch through global
+ * memory and wait for one another.  The waits are bounded; one that runs out
+ * leaves NaN in rho and in every observable and state from then on, in each
+ * right-hand side that lacks a value, and raises LIME_FLAG_TIMEOUT in the
+ * status word of lime_redfield_rk4_f64_status.
  */
 typedef struct {
   int32_t n, n_rhs, n_steps, n_obs, obs_every, states_every;
@@ -238,6 +242,14 @@ typedef struct {
 
 size_t lime_redfield_rk4_f64_workspace(int32_t n, int32_t n_rhs);
 int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream);
+/* The same with a device status word (LIME_FLAG_TIMEOUT is ORed into it; may
+ * be NULL) and the number of polls of a wait (0: the default, about two
+ * seconds). */
+int lime_redfield_rk4_f64_status(const LimeRedfieldRK4Desc* d, int32_t* status, uint32_t max_wait, void* stream);
+/* Test infrastructure: the same with one CTA left out, so that the others'
+ * waits run out after max_wait polls; LIME_ERR_UNSUPPORTED for sizes whose
+ * run has no such waits. */
+int lime_redfield_wait_selftest(const LimeRedfieldRK4Desc* d, int32_t* status, uint32_t max_wait, void* stream);
 
 /* The assembly step of lime_redfield_build_f64 alone, from caller-supplied
  * factors (for a differentiable generator whose factors the caller builds

@@ -259,6 +259,8 @@ SIGNATURES = [
     ('lime_redfield_adjoint_split', c_int32, [ctypes.POINTER(RedfieldAdjointSplitDesc), c_void_p]),
     ('lime_redfield_rk4_f64_workspace', c_size_t, [c_int32, c_int32]),
     ('lime_redfield_rk4_f64', c_int32, [ctypes.POINTER(RedfieldRK4Desc), c_void_p]),
+    ('lime_redfield_rk4_f64_status', c_int32, [ctypes.POINTER(RedfieldRK4Desc), c_void_p, ctypes.c_uint32, c_void_p]),
+    ('lime_redfield_wait_selftest', c_int32, [ctypes.POINTER(RedfieldRK4Desc), c_void_p, ctypes.c_uint32, c_void_p]),
     ('lime_redfield_split_workspace', c_size_t, [c_int32, c_int32, c_int32]),
     ('lime_redfield_rk4_split', c_int32, [ctypes.POINTER(RedfieldSplitDesc), c_void_p]),
     ('lime_redfield_split3_workspace', c_size_t, [c_int32, c_int32, c_int32]),

@@ -179,7 +179,8 @@ extern "C" size_t lime_redfield_rk4_f64_workspace(int32_t n, int32_t n_rhs) {
 
 // The time loop in single launches: a chunk is as many steps as the kept
 // states have slots for, and at most about a tenth of a second of FP64 work.
-static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, cudaStream_t st) {
+static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, int32_t* status, uint32_t max_wait,
+                   cudaStream_t st) {
   const int n = d->n, D = n * n, R = d->n_rhs;
   const size_t DR = (size_t)D * R;
   const int obs_every = d->obs_every > 0 ? d->obs_every : 1;
@@ -190,6 +191,7 @@ static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, cudaStre
   r.ws = reinterpret_cast<double2*>(d->workspace) + 3 * DR;
   r.states = reinterpret_cast<double2*>(d->states); r.states_every = d->states_every;
   r.obs_every = d->n_obs > 0 ? obs_every : 0;
+  r.status = status; r.max_wait = max_wait > 0 ? max_wait : rfv::kPollLimit;
   // the caller's states serve the observables when they are the same steps
   const bool own = d->n_obs > 0 && !(d->states && d->states_every == obs_every);
   double2* out = reinterpret_cast<double2*>(d->obs_out);
@@ -215,7 +217,8 @@ static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, cudaStre
   return LIME_OK;
 }
 
-extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream) {
+// withhold: the plan lacks its last CTA, whose words the others wait for
+static int rk4_f64(const LimeRedfieldRK4Desc* d, int32_t* status, uint32_t max_wait, bool withhold, void* stream) {
   if (!d || d->n <= 0 || d->n_rhs <= 0 || d->n_steps < 0 || d->n_obs < 0) return LIME_ERR_ARG;
   if (!d->R || !d->rho || !d->workspace) return LIME_ERR_ARG;
   if (d->n_obs > 0 && (!d->obs_ops || !d->obs_out)) return LIME_ERR_ARG;
@@ -234,8 +237,14 @@ extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream)
     LIME_CUDA_TRY(cudaGetDevice(&dev));
     LIME_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     rfv::Plan plan;
-    if (rfv::plan(D, R, sms, &plan)) return rk4_vec(d, plan, st);
+    const bool one = rfv::plan(D, R, sms, &plan);
+    if (withhold) {
+      if (!one || plan.mode != rfv::kGrid) return LIME_ERR_UNSUPPORTED;
+      --plan.ctas;
+    }
+    if (one) return rk4_vec(d, plan, status, max_wait, st);
   }
+  if (withhold) return LIME_ERR_UNSUPPORTED;
   double2* P = reinterpret_cast<double2*>(d->rho);
   double2* acc = reinterpret_cast<double2*>(d->workspace);
   double2* S0 = acc + DR;
@@ -268,4 +277,19 @@ extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream)
   }
   count_launch(launches);
   return LIME_OK;
+}
+
+extern "C" int lime_redfield_rk4_f64(const LimeRedfieldRK4Desc* d, void* stream) {
+  return rk4_f64(d, nullptr, 0, false, stream);
+}
+
+extern "C" int lime_redfield_rk4_f64_status(const LimeRedfieldRK4Desc* d, int32_t* status, uint32_t max_wait,
+                                            void* stream) {
+  return rk4_f64(d, status, max_wait, false, stream);
+}
+
+extern "C" int lime_redfield_wait_selftest(const LimeRedfieldRK4Desc* d, int32_t* status, uint32_t max_wait,
+                                           void* stream) {
+  if (!status || max_wait == 0) return LIME_ERR_ARG;
+  return rk4_f64(d, status, max_wait, true, stream);
 }

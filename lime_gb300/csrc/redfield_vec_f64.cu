@@ -13,7 +13,9 @@
 //             word {value, stage number}, so the reader polls the data itself
 //             and no fence or barrier stands between writer and reader.  The
 //             launch is cooperative (all CTAs resident), the polls are
-//             bounded; a wait that runs out leaves NaN in the state.
+//             bounded.  A CTA whose wait runs out raises LIME_FLAG_TIMEOUT
+//             and leaves NaN in its part of the state and of every state
+//             that the launch should still have kept.
 // Two buffers suffice: a CTA writes the input of stage s + 2 only after it
 // has read all of stage s + 1, which its owners wrote after reading all of s.
 //
@@ -40,6 +42,8 @@ struct Args {
   ulonglong2* xch;       // [2][F]
   double2* states;
   double2* hist;
+  int32_t* status;
+  uint32_t max_wait;
 };
 
 __device__ __forceinline__ ulonglong2 ld_tagged(const ulonglong2* p) {
@@ -68,8 +72,7 @@ __device__ __forceinline__ double flip(double x, int mask) {
   return __hiloint2double(__double2hiint(x) ^ mask, __double2loint(x));
 }
 
-constexpr int kPoll = 4;                     // words a thread has in flight
-constexpr long long kPollLimit = 1 << 21;    // polls of one batch (about two seconds)
+constexpr int kPoll = 4;   // words a thread has in flight
 
 template <int kMode>
 __global__ void __launch_bounds__(kThreads, 1) rk4_kernel(Args a) {
@@ -120,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, 1) rk4_kernel(Args a) {
         const ulonglong2* src = a.xch + (size_t)(tag & 1) * F;
         for (int b = t; b < F; b += kThreads * kPoll) {
           ulonglong2 v[kPoll];
-          long long tries = 0;
+          uint32_t tries = 0;
           bool all;
           do {
             all = true;
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1) rk4_kernel(Args a) {
 #pragma unroll
             for (int u = 0; u < kPoll; ++u)
               if (b + u * kThreads < F) all &= v[u].y == tag;
-          } while (!all && ++tries < kPollLimit);
+          } while (!all && ++tries < a.max_wait);
           if (!all) {
             expired = 1;
             break;
@@ -141,8 +144,18 @@ __global__ void __launch_bounds__(kThreads, 1) rk4_kernel(Args a) {
         }
         __syncthreads();
         if (expired) {
-          for (int j = t; j < O; j += kThreads)
-            reinterpret_cast<double*>(a.P)[f0 + j] = __longlong_as_double(0x7ff8000000000000LL);
+          const double nan = __longlong_as_double(0x7ff8000000000000LL);
+          if (t == 0 && a.status != nullptr) atomicOr(a.status, LIME_FLAG_TIMEOUT);
+          for (int j = t; j < O; j += kThreads) {
+            reinterpret_cast<double*>(a.P)[f0 + j] = nan;
+            for (int k = done; k <= a.step0 + a.n_steps; ++k) {
+              if (a.states != nullptr && k % a.states_every == 0)
+                reinterpret_cast<double*>(a.states)[(int64_t)(k / a.states_every - 1) * F + f0 + j] = nan;
+              if (a.hist != nullptr && k % a.obs_every == 0)
+                reinterpret_cast<double*>(a.hist)[(int64_t)(k / a.obs_every - 1 - a.step0 / a.obs_every) * F + f0 + j] =
+                    nan;
+            }
+          }
           return;
         }
       }
@@ -303,6 +316,7 @@ int launch(const Plan& p, const Run& r, int step0, int steps, double2* hist, cud
   a.hist = hist; a.obs_every = r.obs_every > 0 ? r.obs_every : 1;
   a.dt = r.dt; a.sixth = sixth_of(r.dt); a.L = r.L; a.P = r.P;
   a.xch = reinterpret_cast<ulonglong2*>(r.ws);
+  a.status = r.status; a.max_wait = r.max_wait;
   return p.mode == kSolo ? launch_mode<kSolo>(p, a, st)
                          : p.mode == kCluster ? launch_mode<kCluster>(p, a, st) : launch_mode<kGrid>(p, a, st);
 }

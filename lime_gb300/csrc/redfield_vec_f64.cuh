@@ -39,7 +39,10 @@ struct Run {
   double2* states; int states_every;
   // observables: every obs_every steps hist holds the state (the caller evaluates them per chunk)
   int obs_every;         // 0: none
+  int32_t* status;       // LIME_FLAG_TIMEOUT when a wait runs out, or null
+  uint32_t max_wait;     // polls of a wait
 };
+constexpr uint32_t kPollLimit = 1u << 21;   // about two seconds
 
 // runs steps [step0, step0 + steps); hist: slots of D x R, the first one for
 // the first multiple of obs_every after step0

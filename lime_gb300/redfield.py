@@ -124,12 +124,22 @@ def _as_generator(R, device):
     return Rd, n
 
 
+def check_status(status: torch.Tensor):
+    """Raises what the kernels left in the status word of ``propagate_vec``
+    (waits for them)."""
+    flags = int(status.item())
+    if flags:
+        raise nat.KernelFlagError(flags, 'Redfield RK4 (fp64)')
+
+
 def propagate_vec(R, rho0_eb: torch.Tensor, dt: float, n_steps: int, e_eb=None, states_every=0,
-                  obs_every=1):
+                  obs_every=1, status: torch.Tensor | None = None):
     """RK4 of eigenbasis density matrices (B, n, n) under the dense generator.
 
     Returns (obs (B, n_steps // obs_every, n_obs), states (B, S, n, n) or None,
-    final rho (B, n, n)), all in the eigenbasis.
+    final rho (B, n, n)), all in the eigenbasis.  ``status``: a zeroed int32
+    device word for a caller that checks it itself (``check_status``) after
+    several calls or after reading the results; by default it is checked here.
     """
     lib = nat.require_device()
     Rd, n = R
@@ -161,7 +171,11 @@ def propagate_vec(R, rho0_eb: torch.Tensor, dt: float, n_steps: int, e_eb=None, 
         d.obs_ops, d.obs_out = E.data_ptr(), obs.data_ptr()
     d.states = None if states is None else states.data_ptr()
     d.workspace, d.workspace_bytes = ws.data_ptr(), wsb
-    nat.check(lib.lime_redfield_rk4_f64(d, engine._stream_ptr()), 'lime_redfield_rk4_f64')
+    word = torch.zeros(1, dtype=torch.int32, device=dev) if status is None else status
+    nat.check(lib.lime_redfield_rk4_f64_status(d, word.data_ptr(), 0, engine._stream_ptr()),
+              'lime_redfield_rk4_f64_status')
+    if status is None:
+        check_status(word)
     o = obs[:n_slots, :, :n_obs].permute(1, 0, 2)
     st = None
     if states is not None:
@@ -327,9 +341,9 @@ def propagate_vec_split(R, rho0_eb: torch.Tensor, dt: float, n_steps: int, e_eb=
     return o, None, P.reshape(B, n, n)
 
 
-def _propagate(Rg, r0t, dt, Nt, e_eb, states_every=0, precision='fp64'):
+def _propagate(Rg, r0t, dt, Nt, e_eb, states_every=0, precision='fp64', status=None):
     if precision == 'fp64':
-        return propagate_vec(Rg, r0t, dt, Nt, e_eb, states_every=states_every)
+        return propagate_vec(Rg, r0t, dt, Nt, e_eb, states_every=states_every, status=status)
     if precision != 'split':
         raise ValueError("precision must be 'fp64' or 'split'")
     if not states_every:
@@ -395,8 +409,9 @@ def _redfield(R, rho0, evecs=None, Nt=1, dt=0.005, t0=0, e_ops=None, return_resu
                 f.write(fmt.format(t, *rows[k]))
         out = rho.reshape(rho.shape[0], -1).cpu().numpy()
         return out if batched else out[0]
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
     o, st, rho = _propagate(Rg, r0t, dt, Nt, e_eb, states_every=1 if store_states else 0,
-                            precision=precision)
+                            precision=precision, status=status)
     res = Result(dt=dt, Nt=Nt, rho0=rho0, t0=t0, nout=1)
     obs_np = o.cpu().numpy()
     res.observables = obs_np if batched else obs_np[0]
@@ -408,6 +423,7 @@ def _redfield(R, rho0, evecs=None, Nt=1, dt=0.005, t0=0, e_ops=None, return_resu
     else:
         fin = rho if V is None else zl.from_basis(V, rho)
         res.rholist = fin.cpu().numpy() if batched else [fin[0].cpu().numpy()]
+    check_status(status)
     return res
 
 

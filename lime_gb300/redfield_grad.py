@@ -27,7 +27,7 @@ import torch
 
 from . import _native as nat
 from . import engine
-from .redfield import propagate_vec, propagate_vec_split, stage_buffer_floats
+from .redfield import check_status, propagate_vec, propagate_vec_split, stage_buffer_floats
 
 CDT = torch.complex128
 
@@ -122,16 +122,19 @@ class _Propagate(torch.autograd.Function):
                                         device=rho.device)
                 left -= need
         ckpts, parts = [], []
+        status = torch.zeros(1, dtype=torch.int32, device=rho.device)
         for (s0, m), sbuf in zip(segs, stages):
             ckpts.append(rho)
             if precision == 'fp64':
-                o, _, rho = propagate_vec(Rg, rho, dt, m, list(E), obs_every=obs_every)
+                o, _, rho = propagate_vec(Rg, rho, dt, m, list(E), obs_every=obs_every, status=status)
             elif sbuf is not None:
                 o, _, rho = propagate_vec_split(Rg, rho, dt, m, list(E), obs_every=obs_every, stage_out=sbuf)
             else:
                 # the block form: the backward pass recomputes segments with it
                 o, _, rho = propagate_vec_split(Rg, rho, dt, m, list(E), obs_every=obs_every, product='4m')
             parts.append(o)
+        if precision == 'fp64':
+            check_status(status)
         obs = torch.cat(parts, 1) if parts else torch.zeros((rho.shape[0], 0, E.shape[0]), dtype=CDT,
                                                            device=rho.device)
         ctx.save_for_backward(R.detach(), E, *ckpts)
