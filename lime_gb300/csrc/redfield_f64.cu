@@ -178,7 +178,8 @@ extern "C" size_t lime_redfield_rk4_f64_workspace(int32_t n, int32_t n_rhs) {
 }
 
 // The time loop in single launches: a chunk is as many steps as the kept
-// states have slots for, and at most about a tenth of a second of FP64 work.
+// states have slots for, and at most about a tenth of a second by the plan's
+// count of a stage's clocks.
 static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, int32_t* status, uint32_t max_wait,
                    cudaStream_t st) {
   const int n = d->n, D = n * n, R = d->n_rhs;
@@ -198,8 +199,8 @@ static int rk4_vec(const LimeRedfieldRK4Desc* d, const rfv::Plan& plan, int32_t*
   const double2* E = reinterpret_cast<const double2*>(d->obs_ops);
   int rc = rfv::begin(plan, r, st);
   if (rc != LIME_OK) return rc;
-  const double per_step = 16.0 * D * (double)D * R;
-  int64_t chunk = (int64_t)fmax(1.0, fmin((double)d->n_steps, 5e10 / per_step));
+  constexpr double kLaunchClocks = 2e8;
+  int64_t chunk = (int64_t)fmax(1.0, fmin((double)d->n_steps, kLaunchClocks / (4.0 * plan.clocks)));
   if (own && chunk > (int64_t)rfv::kHistory * obs_every) chunk = (int64_t)rfv::kHistory * obs_every;
   for (int64_t s0 = 0; s0 < d->n_steps; s0 += chunk) {
     const int steps = (int)(d->n_steps - s0 < chunk ? d->n_steps - s0 : chunk);

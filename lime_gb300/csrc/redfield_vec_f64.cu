@@ -266,6 +266,7 @@ bool plan(int D, int R, int sms, Plan* out) {
   const double work = 4.0 * (double)D * D * R / 1.68;
   const double solo = work + kSoloCost, cluster = work / kMaxCluster + kClusterCost, grid = work / sms + kGridCost;
   const Mode m = solo <= cluster && solo <= grid ? kSolo : cluster <= grid ? kCluster : kGrid;
+  out->clocks = m == kSolo ? solo : m == kCluster ? cluster : grid;
   return plan_mode(D, R, m, m == kSolo ? 1 : m == kCluster ? kMaxCluster : sms, out);
 }
 

@@ -21,6 +21,7 @@ struct Plan {
   int red;        // lanes that add a team's partial sums
   int l_smem;     // the CTA's rows of the generator are kept in shared memory
   size_t smem;
+  double clocks;  // of a stage, predicted
 };
 
 // shapes whose stage input fits the shared memory of an SM beside the rest

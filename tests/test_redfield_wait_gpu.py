@@ -83,3 +83,16 @@ def test_no_waits_to_expire(lib):
         d.R, d.rho = L.data_ptr(), rho.data_ptr()
         d.workspace, d.workspace_bytes = ws.data_ptr(), size
         assert lib.lime_redfield_wait_selftest(d, word.data_ptr(), POLLS, None) == -2
+
+
+@pytest.mark.parametrize('n,steps,fixed', [(2, 120000, 900), (6, 60000, 1700), (14, 30000, 3600)])
+def test_launches_are_bounded(lib, n, steps, fixed):
+    """A stage takes at least its mode's fixed clocks; 2e8 of them are a launch."""
+    from lime_gb300 import redfield
+    D = n * n
+    L = torch.zeros(D, D, dtype=torch.complex128, device='cuda')
+    rho = torch.ones(1, n, n, dtype=torch.complex128, device='cuda')
+    before = nat.launch_count()
+    _, _, fin = redfield.propagate_vec((L, n), rho, 0.05, steps)
+    assert nat.launch_count() - before >= 4 * steps * fixed / 2e8
+    assert torch.equal(fin, rho)
