@@ -53,9 +53,11 @@ def _host_or_device(a, device):
     """A host operator as a dense complex128 array, a device tensor on ``device``."""
     if isinstance(a, torch.Tensor) and a.device.type != 'cpu':
         return as_device(a, device)
-    if isinstance(a, torch.Tensor):
-        a = a.detach().resolve_conj()
-    return np.asarray(_to_dense_np(a), dtype=np.complex128)
+    if type(a) is np.ndarray and a.dtype == np.complex128 and a.flags.c_contiguous:
+        return a
+    # torch's conversion, so that the same operators are taken as for the
+    # device: types that NumPy lacks, lazily conjugated or negated views
+    return as_device(a, 'cpu').detach().resolve_conj().resolve_neg().numpy()
 
 
 class DiagonalOps:
