@@ -250,7 +250,11 @@ class LindbladGenerator:
         gen = LindbladGenerator(n=n, P=P, heff=heff, m=(m if lg is not None or rate is not None else None),
                                 l_dense=ld, k_dense=d.k_dense, shared=shared)
         if gen.m is not None and m_diagonal:
-            gen.split_cache['m_diagonal'] = True   # M = diag(rates), or one entry an operator
+            if lg is None:
+                gen.split_cache['m_diagonal'] = True   # site dephasing alone: M = diag(rates)
+            else:
+                # one entry an operator: of this tensor, as long as nothing is written to it
+                gen.split_cache['m_built_diagonal'] = (gen.m, gen.m._version)
         return gen
 
 
@@ -361,7 +365,9 @@ def split_supported(gen: LindbladGenerator) -> str | None:
 
 def m_is_diagonal(gen: LindbladGenerator) -> bool:
     """Whether M is diagonal (known from the operators, or a test on the device)."""
-    return bool(gen.split_cache.get('m_diagonal')) or is_diagonal(gen.m)
+    built, version = gen.split_cache.get('m_built_diagonal', (None, 0))
+    return bool(gen.split_cache.get('m_diagonal')) or (built is gen.m and version == gen.m._version) \
+        or is_diagonal(gen.m)
 
 
 def _pow2_exponent(target: float, bound: float) -> int:
