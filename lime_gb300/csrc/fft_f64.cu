@@ -29,10 +29,11 @@ constexpr int kMaxPow2 = 8192;
 constexpr int kRoots = kMaxPow2 / 2;
 
 // exp(-2 pi i j / 8192), j = 0 .. 4095, from the Taylor series of the first
-// octant in 62-bit fixed point (error under 2^-59), rounded once
-struct Roots {
+// octant in 62-bit fixed point (error under 2^-59), rounded once; read as double2
+struct alignas(sizeof(double2)) Roots {
   double v[2 * kRoots];
 };
+static_assert(alignof(Roots) >= alignof(double2), "root() loads 16 bytes at a time");
 constexpr long long fixmul(long long a, long long b) { return (long long)(((__int128)a * b) >> 62); }
 constexpr Roots make_roots() {
   Roots r{};
