@@ -532,7 +532,8 @@ static RK4Plan plan_rk4(int n, int c, int k_dense) {
   const int64_t nn = (int64_t)n * n;
   P.cluster = c;
   const int64_t per = (nn + P.cluster - 1) / P.cluster;
-  P.e = per <= kMaxThreads ? 1 : per <= 2 * kMaxThreads ? 2 : per <= 4 * kMaxThreads ? 4 : per <= 8 * kMaxThreads ? 8 : 0;
+  const int64_t items = (per + kMaxThreads - 1) / kMaxThreads;
+  P.e = items <= 1 ? 1 : items <= 2 ? 2 : items <= 4 ? 4 : items <= 8 ? 8 : 0;
   if (n > 65535 || (P.cluster == 1 && n > 64)) P.e = 0;
   P.nt = P.e == 0 ? kMaxThreads : (int)(((per + P.e - 1) / P.e + 31) / 32 * 32);
   if (k_dense > 0 && P.nt < 128) P.nt = 128;   // threads without an item still form rows of Y

@@ -883,7 +883,8 @@ __global__ void __launch_bounds__(kThreads, 2) lindblad_rk4_split_kernel(Args a)
 #pragma unroll
       for (int jj = 0; jj < kCols; ++jj) {
         const int j = j0 + jj;
-        const double v = fpconv::scale_pow2(fpconv::widen_f32(at(rho, jj)) + fpconv::widen_f32(S.rlo[j * 128 + r]), ebi);
+        const double v =
+            fpconv::scale_pow2(fpconv::widen_f32(at(rho, jj)) + fpconv::widen_f32(S.rlo[j * 128 + r]), ebi);
         if (!isfinite(at(rho, jj))) flags |= LIME_FLAG_NONFINITE;
         sd[2 * stage_index(i, j) + comp] = fpconv::from_bits64(fpconv::bits64(v) ^ neg);
       }
@@ -1386,7 +1387,8 @@ __global__ void __launch_bounds__(128, (SmallShape<kW, kDual>::kCtas)) lindblad_
       const uint64_t neg = is_re ? 0ull : 0x8000000000000000ull;
 #pragma unroll
       for (int jj = 0; jj < kC; ++jj) {
-        const double v = fpconv::scale_pow2(fpconv::widen_f32(at(rho, jj)) + fpconv::widen_f32(S.rlo[jj * 128 + t]), ebi);
+        const double v =
+            fpconv::scale_pow2(fpconv::widen_f32(at(rho, jj)) + fpconv::widen_f32(S.rlo[jj * 128 + t]), ebi);
         if (!isfinite(at(rho, jj))) flags |= LIME_FLAG_NONFINITE;
         sd[2 * pos(i, j0 + jj) + comp] = fpconv::from_bits64(fpconv::bits64(v) ^ neg);
       }
@@ -1637,9 +1639,14 @@ extern "C" int lime_lindblad_rk4_split(const LimeLindbladSplitDesc* d, void* str
   int threads = split::kThreads, resident = 2;
   if (!driven && d->n <= 32) {
     const bool w16 = d->n <= 16;
-    const bool dual = d->batch <= (w16 ? split::SmallShape<16, true>::kCtas : split::SmallShape<32, true>::kCtas) * g_num_sms;
-    kern = w16 ? (dual ? split::lindblad_rk4_split_small_kernel<16, true> : split::lindblad_rk4_split_small_kernel<16, false>)
-               : (dual ? split::lindblad_rk4_split_small_kernel<32, true> : split::lindblad_rk4_split_small_kernel<32, false>);
+    const int both = w16 ? split::SmallShape<16, true>::kCtas : split::SmallShape<32, true>::kCtas;
+    const bool dual = d->batch <= both * g_num_sms;
+    if (w16)
+      kern = dual ? split::lindblad_rk4_split_small_kernel<16, true>
+                  : split::lindblad_rk4_split_small_kernel<16, false>;
+    else
+      kern = dual ? split::lindblad_rk4_split_small_kernel<32, true>
+                  : split::lindblad_rk4_split_small_kernel<32, false>;
     smem = (w16 ? sizeof(split::SmallSmem<16>) : sizeof(split::SmallSmem<32>)) + 128;
     threads = 128;
     resident = w16 ? (dual ? split::SmallShape<16, true>::kCtas : split::SmallShape<16, false>::kCtas)

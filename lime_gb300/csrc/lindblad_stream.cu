@@ -191,7 +191,8 @@ __device__ __forceinline__ void fused_epilogue(const Args& a, int b, int mt, int
       const int R = mt * kBM + dl;
       const size_t xo = (size_t)b * inst_floats(a) + (size_t)(nt * kBN + jl) * np + R;
       const int jj = nt * kBN + jl, x = jj >= np ? jj - np : jj;
-      if (R < rows_x && x < rows_x && in_bounds(xo * sizeof(float), 8 * sizeof(float), a.st_floats * sizeof(float), a.status)) {
+      if (R < rows_x && x < rows_x &&
+          in_bounds(xo * sizeof(float), 8 * sizeof(float), a.st_floats * sizeof(float), a.status)) {
         float v[8];
         park8(jl, dl, v);
         sg::st8(a.Xg + xo, v);
@@ -1060,8 +1061,9 @@ int lsm_prepare(const LimeLindbladStreamDesc* d, LsmRun& r, cudaStream_t st, int
   r.heff_t = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(d->workspace) + L.total);
 
   const int per_g = L.MT1 * 128 + (K > 0 ? L.MT2 * 128 : 0);
-  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(reinterpret_cast<const double2*>(d->heff), d->heff_stride,
-                                                  reinterpret_cast<const double2*>(d->l_ops), d->l_stride, a, co, 0);
+  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(
+      reinterpret_cast<const double2*>(d->heff), d->heff_stride, reinterpret_cast<const double2*>(d->l_ops),
+      d->l_stride, a, co, 0);
   LIME_CUDA_TRY(cudaGetLastError());
   ++launches;
   a.B1n[0] = r.B1[0][0]; a.B1n[1] = r.B1[0][1];
@@ -1129,11 +1131,11 @@ int lsm_observe(const LimeLindbladStreamDesc* d, LsmRun& r, int step, cudaStream
     double2* out = reinterpret_cast<double2*>(d->obs_out);
     const int slots = d->n_steps / obs_every, slot = (step + 1) / obs_every - 1;
     if (d->obs_diag)
-      LIME_TRY(launch_chained(lsm::observe_diag_kernel,
-                              (unsigned)(((int64_t)r.B * d->n_obs + 3) / 4), 128, 0, st, r.a, E, d->obs_stride, d->n_obs, r.B, out, slots, slot));
+      LIME_TRY(launch_chained(lsm::observe_diag_kernel, (unsigned)(((int64_t)r.B * d->n_obs + 3) / 4), 128, 0, st,
+                              r.a, E, d->obs_stride, d->n_obs, r.B, out, slots, slot));
     else
-      LIME_TRY(launch_chained(lsm::observe_kernel,
-                              r.B * d->n_obs, lsm::kObsThreads, 0, st, r.a, E, d->obs_stride, d->n_obs, out, slots, slot));
+      LIME_TRY(launch_chained(lsm::observe_kernel, r.B * d->n_obs, lsm::kObsThreads, 0, st, r.a, E, d->obs_stride,
+                              d->n_obs, out, slots, slot));
     ++launches;
   }
   return LIME_OK;
@@ -1172,8 +1174,8 @@ extern "C" int lime_lindblad_rk4_stream(const LimeLindbladStreamDesc* d, void* s
                                              reinterpret_cast<const double2*>(d->drive_ops),
                                              d->drive_coef + (size_t)step * d->n_drive, d->n_drive, r.heff_t);
       LIME_CUDA_TRY(cudaGetLastError());
-      lsm::convert_kernel<<<G * L.np, lsm_convert_threads(L), 0, st>>>(r.heff_t, G == 1 ? 0 : (int64_t)d->n * d->n, nullptr, 0, a,
-                                                    r.co, 1);
+      lsm::convert_kernel<<<G * L.np, lsm_convert_threads(L), 0, st>>>(
+          r.heff_t, G == 1 ? 0 : (int64_t)d->n * d->n, nullptr, 0, a, r.co, 1);
       LIME_CUDA_TRY(cudaGetLastError());
       launches += 2;
     }
@@ -1229,10 +1231,10 @@ extern "C" int lime_lindblad_rk4_stream_groups(const LimeLindbladStreamDesc* des
   LIME_CUDA_TRY(cudaGetDevice(&dev));
   LIME_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const size_t smem = sg::kSmemBytes;
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<false, lsm::kMaxGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<true, lsm::kMaxGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<false, lsm::kMaxGroups>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  LIME_CUDA_TRY(cudaFuncSetAttribute(lsm::gemm_groups_kernel<true, lsm::kMaxGroups>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // tile lists: groups by decreasing chunks per tile (order 1), or as given (order 0)
   int ord1[lsm::kMaxGroups], ord2[lsm::kMaxGroups];
   int n2 = 0;
@@ -1394,8 +1396,8 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
   int64_t launches = 0;
 
   const int per_g = L.MT1 * 128;
-  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(reinterpret_cast<const double2*>(d->heff), d->heff_stride,
-                                                  nullptr, 0, af, cf, 0);
+  lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(
+      reinterpret_cast<const double2*>(d->heff), d->heff_stride, nullptr, 0, af, cf, 0);
   LIME_CUDA_TRY(cudaGetLastError());
   lsm::convert_kernel<<<G * per_g, lsm_convert_threads(L), 0, st>>>(reinterpret_cast<const double2*>(d->heff_adj),
                                                   d->heff_adj_stride, nullptr, 0, aa, ca, 0);
@@ -1450,7 +1452,9 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
       aa.B1n[0] = B1[c][0]; aa.B1n[1] = B1[c][1];
       aa.Sn = Sbuf[c];
       LIME_TRY(launch_chained(lsm::adj_source_kernel, eb, 256, 0, st, aa, J, B,
-                              reinterpret_cast<const double2*>(d->obs_ops), d->obs_stride, d->n_obs, reinterpret_cast<const double2*>(d->obs_grad), n_slots, slot, reinterpret_cast<const float2*>(d->obs_coef)));
+                              reinterpret_cast<const double2*>(d->obs_ops), d->obs_stride, d->n_obs,
+                              reinterpret_cast<const double2*>(d->obs_grad), n_slots, slot,
+                              reinterpret_cast<const float2*>(d->obs_coef)));
       LIME_TRY(launch_chained(lsm::adj_scale_kernel, 1, 1, 0, st, J));
       LIME_TRY(launch_chained(lsm::adj_start_kernel, eb, 256, 0, st, aa, J, B, (float)(dt / 6.0)));
       launches += 3;
@@ -1461,8 +1465,9 @@ extern "C" int lime_lindblad_adjoint_stream(const LimeLindbladAdjointStreamDesc*
         aa.Sn = Sbuf[c ^ 1];
         grc = lsm_gemm<false>(aa, gemm_grid, sms, st);
         if (grc != LIME_OK) return grc;
-        LIME_TRY(launch_chained(lsm::adj_grad_kernel,
-                                B * ((d->n + 7) / 8), lsm::kGradThreads, 0, st, aa, Sbuf[c], store + ((size_t)s * 4 + (i - 1)) * B * inst, d->grad_diag, d->grad_bond, d->grad_gamma));
+        LIME_TRY(launch_chained(lsm::adj_grad_kernel, B * ((d->n + 7) / 8), lsm::kGradThreads, 0, st, aa, Sbuf[c],
+                                store + ((size_t)s * 4 + (i - 1)) * B * inst, d->grad_diag, d->grad_bond,
+                                d->grad_gamma));
         const float c_l = (float)(i == 2 ? dt / 6.0 : dt / 3.0);
         const float c_y = (float)(i == 4 ? dt : dt / 2.0);
         LIME_TRY(launch_chained(lsm::adj_finish_kernel, tb, 256, 0, st, aa, J, i, c_l, c_y));

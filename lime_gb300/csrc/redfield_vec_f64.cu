@@ -249,8 +249,8 @@ static bool plan_mode(int D, int R, Mode mode, int ctas, Plan* P) {
   int g = 1;
   while (g < 16 && 2 * g <= T && 2 * g * P->outs <= kThreads) g <<= 1;
   P->red = g;
-  const size_t base = ((size_t)(mode == kCluster ? 2 : 1) * F + ((P->outs > kThreads ? P->outs : kThreads) + 1) / 2 * 2 +
-                       2 * (size_t)P->outs) * 8;
+  const int parts = ((P->outs > kThreads ? P->outs : kThreads) + 1) / 2 * 2;
+  const size_t base = ((size_t)(mode == kCluster ? 2 : 1) * F + parts + 2 * (size_t)P->outs) * 8;
   const size_t rows = (size_t)(P->outs + 2 * R - 2) / (2 * R) + 1;
   const size_t lb = rows * D * 16;
   if (base > kSmemMax) return false;

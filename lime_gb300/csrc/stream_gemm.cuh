@@ -75,7 +75,7 @@ static_assert(kCK % 16 == 0 && 128 % kCK == 0, "K chunks are whole MMA K steps a
 
 struct __align__(1024) Smem {
   uint8_t stage[kStages][5][kPiece];               // A0 A1 A2 B0 B1; the parked tile after the last MMA
-  float lo[kBN * kBM];                             // parked tile of a sequence, or its low words (park_split), [col][row]
+  float lo[kBN * kBM];                             // parked tile of a sequence or low words (park_split), [col][row]
   uint64_t full[kStages], empty[kStages], accf[2], acce[2], drain;
   uint32_t tmem_base;
   int abort;
@@ -231,8 +231,7 @@ struct Tile {
 // 1175 us of the 9216-dimensional Redfield stage run alone) is the issue
 // slots of these additions, so they are packed two to an instruction and
 // both words stay in registers: 1175 -> 961 us.  (Copies are not the bound:
-// leaving them out, or halving the L2 reads by cluster multicast, changes
-// nothing.)
+// leaving them out, or halving the L2 reads, changes nothing.)
 __device__ __forceinline__ void drain_group(uint32_t d0, float (&hi)[kEpiCols], float (&lo)[kEpiCols]) {
 #pragma unroll
   for (int q = 0; q < kEpiCols / 8; ++q) {
