@@ -13,9 +13,13 @@
 //
 // Bound: the FP64 pipe (1.68 lanes per clock and SM; everything else is
 // nearly free beside it), so the butterflies are counted in FP64
-// instructions: u + w v and 2 u - (u + w v) are 6 fma, the first pass's
-// factors 1 and -i are 4 additions, and the factors come from a table that
-// the compiler fills (a sincospi in each butterfly took 40 of 48).  256
+// instructions: u + w v and u - w v are 8 fma, or 6 where the second is
+// 2 u - (u + w v); the first pass's factors 1 and -i are 4 additions, and the
+// factors come from a table that the compiler fills (a sincospi in each
+// butterfly took 40 of 48).  The 6-fma form in all stages leaves an rms error
+// 4 to 5 % above that of u +- t with a rounded t = w v, the 8-fma form one 3 to
+// 4 % below; the first stage of a pass takes the former, the two others the
+// latter, and the error is at or below the one of u +- t at every length.  256
 // transforms of 4096: 722 -> 93 us, 33.5 + 4 FP64 instructions a point being
 // 78 us; 100 of length 999: 504 -> 51 us in the transforms, 3 launches for 6.
 
@@ -78,6 +82,12 @@ __device__ __forceinline__ int sw(int i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i
 
 // (u, v) <- (u + w v, u - w v)
 __device__ __forceinline__ void bfly(double2& u, double2& v, double2 w) {
+  const double2 r = make_double2(fma(-w.y, v.y, fma(w.x, v.x, u.x)), fma(w.y, v.x, fma(w.x, v.y, u.y)));
+  v = make_double2(fma(w.y, v.y, fma(-w.x, v.x, u.x)), fma(-w.y, v.x, fma(-w.x, v.y, u.y)));
+  u = r;
+}
+// the same with 6 instructions for 8; the second result takes over the first one's rounding error
+__device__ __forceinline__ void bfly_6(double2& u, double2& v, double2 w) {
   const double2 r = make_double2(fma(-w.y, v.y, fma(w.x, v.x, u.x)), fma(w.y, v.x, fma(w.x, v.y, u.y)));
   v = make_double2(fma(2.0, u.x, -r.x), fma(2.0, u.y, -r.y));
   u = r;
@@ -156,7 +166,7 @@ __device__ void transform(double2* s, int L, const Load& load, const Store& stor
 #pragma unroll
       for (int m = 0; m < 8; ++m) v[m] = s[sw(base + (m << lh))];
 #pragma unroll
-      for (int m = 0; m < 8; m += 2) bfly(v[m], v[m + 1], w1);
+      for (int m = 0; m < 8; m += 2) bfly_6(v[m], v[m + 1], w1);
 #pragma unroll
       for (int m = 0; m < 8; m += 4) {
         bfly(v[m], v[m + 2], w2);
