@@ -139,7 +139,8 @@ def propagate_vec(R, rho0_eb: torch.Tensor, dt: float, n_steps: int, e_eb=None, 
     Returns (obs (B, n_steps // obs_every, n_obs), states (B, S, n, n) or None,
     final rho (B, n, n)), all in the eigenbasis.  ``status``: a zeroed int32
     device word for a caller that checks it itself (``check_status``) after
-    several calls or after reading the results; by default it is checked here.
+    several calls or after reading the results; by default it is checked here,
+    except under stream capture.
     """
     lib = nat.require_device()
     Rd, n = R
@@ -174,7 +175,7 @@ def propagate_vec(R, rho0_eb: torch.Tensor, dt: float, n_steps: int, e_eb=None, 
     word = torch.zeros(1, dtype=torch.int32, device=dev) if status is None else status
     nat.check(lib.lime_redfield_rk4_f64_status(d, word.data_ptr(), 0, engine._stream_ptr()),
               'lime_redfield_rk4_f64_status')
-    if status is None:
+    if status is None and not torch.cuda.is_current_stream_capturing():
         check_status(word)
     o = obs[:n_slots, :, :n_obs].permute(1, 0, 2)
     st = None

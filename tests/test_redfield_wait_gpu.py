@@ -96,3 +96,17 @@ def test_launches_are_bounded(lib, n, steps, fixed):
     _, _, fin = redfield.propagate_vec((L, n), rho, 0.05, steps)
     assert nat.launch_count() - before >= 4 * steps * fixed / 2e8
     assert torch.equal(fin, rho)
+
+
+@pytest.mark.parametrize('n', [2, 6, 14])
+def test_captured_call(lib, n):
+    """A call recorded in a graph reads nothing back and replays."""
+    from lime_gb300 import redfield
+    L, rho, E = _inputs(n, 1)
+    want = redfield.propagate_vec((L, n), rho, 0.05, 5, E)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = redfield.propagate_vec((L, n), rho, 0.05, 5, E)
+    for _ in range(2):
+        graph.replay()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
