@@ -73,6 +73,18 @@ __global__ void __launch_bounds__(128) zgemm_element_kernel(Args a, int64_t tota
   }
 }
 
+// Addresses of a strided operand, [lo, hi] in elements.
+struct Span {
+  const double2 *lo, *hi;
+};
+static Span span(const double2* p, int64_t d0, int64_t s0, int64_t d1, int64_t s1, int64_t d2, int64_t s2) {
+  Span r{p, p};
+  const int64_t len[3] = {(d0 - 1) * s0, (d1 - 1) * s1, (d2 - 1) * s2};
+  for (int64_t v : len) (v < 0 ? r.lo : r.hi) += v;
+  return r;
+}
+static bool meets(const Span& a, const Span& b) { return a.lo <= b.hi && b.lo <= a.hi; }
+
 }  // namespace zg
 }  // namespace lime
 
@@ -94,10 +106,16 @@ extern "C" int lime_zgemm_strided_f64(const LimeZgemmDesc* d, void* stream) {
   const unsigned gy = (unsigned)((d->M + rf::kTile - 1) / rf::kTile);
   if (gy > 65535u) return LIME_ERR_UNSUPPORTED;
   // elements: while the tiles hold more than twice the outputs, or leave
-  // most SMs without one (fewer than 76 tiles: an SM's share of elements is
-  // then the smaller)
+  // most SMs without one (fewer than 76 tiles, half of the 152 SMs: an SM's
+  // share of elements is then the smaller).  Not where C lies over an operand:
+  // a tile reads all of its operands before it writes (C = A B in the place of
+  // A works up to 64 x 64), an element's thread would write while others read.
   const int64_t outputs = (int64_t)d->M * d->N * d->batch, tiles = (int64_t)gx * gy * d->batch;
-  if (tiles * rf::kTile * rf::kTile > 2 * outputs || tiles < 76) {
+  const zg::Span c = zg::span(a.C, a.M, a.c_rs, a.N, a.c_cs, d->batch, a.c_bs);
+  const bool apart = !zg::meets(c, zg::span(a.A, a.M, a.a_rs, a.K, a.a_cs, d->batch, a.a_bs)) &&
+                     !zg::meets(c, zg::span(a.B, a.K, a.b_rs, a.N, a.b_cs, d->batch, a.b_bs)) &&
+                     !(a.S && zg::meets(c, zg::span(a.S, a.K, a.s_ks, d->batch, a.s_bs, 1, 0)));
+  if (apart && (tiles * rf::kTile * rf::kTile > 2 * outputs || tiles < 76)) {
     const int64_t blocks = (outputs + 127) / 128;
     zg::zgemm_element_kernel<<<(unsigned)(blocks < 1 << 20 ? blocks : 1 << 20), 128, 0, st>>>(a, outputs);
     LIME_CUDA_TRY(cudaGetLastError());
