@@ -96,7 +96,11 @@ __device__ __forceinline__ void rhs_items(const Rows& R, const double2 (&c)[kN],
     f[u] = fma(-c[u].y, flip(ldd<kCg>(xq + oth(u)), sgn(u)), c[u].x * ldd<kCg>(xq + (1 - oth(u))));
   }
   if (R.dense) {
-    // entry e: columns e + (e >= p) and e + (e >= q)
+    // entry e: columns e + (e >= p) and e + (e >= q); h rho and rho h^dag in
+    // sums of their own (one chain of both has 1.4 times the rounding error)
+    double g[kN];
+#pragma unroll
+    for (int u = 0; u < kN; ++u) g[u] = 0.0;
     if (R.real) {
       const double* h = reinterpret_cast<const double*>(R.ent);
 #pragma unroll(kN == 1 ? 4 : 2)
@@ -106,7 +110,7 @@ __device__ __forceinline__ void rhs_items(const Rows& R, const double2 (&c)[kN],
         for (int u = 0; u < kN; ++u) {
           const int p = it[u].p, q = it[u].q;
           f[u] = fma(he[p], flip(ldd<kCg>(x + (Idx)(e + (e >= p)) * ld2 + 2 * q + oth(u)), sgn(u)), f[u]);
-          f[u] = fma(-he[q], flip(ldd<kCg>(x + (Idx)p * ld2 + 2 * (e + (e >= q)) + oth(u)), sgn(u)), f[u]);
+          g[u] = fma(-he[q], flip(ldd<kCg>(x + (Idx)p * ld2 + 2 * (e + (e >= q)) + oth(u)), sgn(u)), g[u]);
         }
       }
     } else {
@@ -121,11 +125,13 @@ __device__ __forceinline__ void rhs_items(const Rows& R, const double2 (&c)[kN],
           const double2 z = ldz<kCg>(reinterpret_cast<const double2*>(x + (Idx)p * ld2 + 2 * (e + (e >= q))));
           f[u] = fma(a.x, flip(it[u].im ? r.x : r.y, sgn(u)), f[u]);
           f[u] = fma(a.y, it[u].im ? r.y : r.x, f[u]);
-          f[u] = fma(-b.x, flip(it[u].im ? z.x : z.y, sgn(u)), f[u]);
-          f[u] = fma(b.y, it[u].im ? z.y : z.x, f[u]);
+          g[u] = fma(-b.x, flip(it[u].im ? z.x : z.y, sgn(u)), g[u]);
+          g[u] = fma(b.y, it[u].im ? z.y : z.x, g[u]);
         }
       }
     }
+#pragma unroll
+    for (int u = 0; u < kN; ++u) f[u] += g[u];
   } else if (R.real) {
 #pragma unroll(kN == 1 ? 2 : 1)
     for (int e = 0; e < W; ++e) {
