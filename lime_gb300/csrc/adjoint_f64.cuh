@@ -29,7 +29,7 @@ struct AdjArgs {
 // workspace per instance, n x n complex matrices: the segment's states and
 // the work matrices of either kernel
 __host__ __device__ inline int64_t adj_ws_mats(int seg_steps, int k_dense) {
-  return (int64_t)seg_steps + 9 + (k_dense > 0 ? 2 : 0);
+  return (int64_t)seg_steps + (k_dense > 0 ? 11 : 10);
 }
 
 // one segment without dense operators (lindblad_adjoint_rows_f64.cu)

@@ -6,10 +6,13 @@
 // their nonzero entries, element by element of the upper triangle and one
 // real component at a time (rows_f64.cuh).  Per step: the three stage states
 // again, four adjoint stages, and per stage the products that the gradients
-// sum; those stay per element over the whole segment and are added up once
-// at its end.  The states and adjoint stage inputs are full matrices, double
-// buffered so that a stage costs one barrier, in shared memory as far as
-// they fit (n up to 41), else in the caller's workspace.
+// sum.  Those are added per element over a step, the steps' sums per element
+// over the segment, and the elements once at its end: one sum per element
+// over all stages has up to 1.3 times the rounding error of sums by rows at
+// each stage, the two levels have 0.7 to 1.05 times.  The states and adjoint
+// stage inputs are full matrices, double buffered so that a stage costs one
+// barrier, in shared memory as far as they fit (n up to 41), else in the
+// caller's workspace.
 //
 // Measured against tiled GEMMs of the full Heff in every stage, with the
 // gradient sums in n threads: 32 matrices of 25 levels, 16 steps, 7.35 -> 0.57
@@ -44,7 +47,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
   const double2* madj = a.m_adj ? a.m_adj + p * a.m_adj_stride : nullptr;
   const double2* obs_ops = a.obs_ops ? a.obs_ops + p * a.obs_stride : nullptr;
   double2* seg = a.ws + (int64_t)b * adj_ws_mats(a.seg_steps, 0) * nn;   // rho_{step0 + s}, s < seg_steps
-  double2* ws = seg + (int64_t)a.seg_steps * nn;                        // 9 matrices
+  double2* ws = seg + (int64_t)a.seg_steps * nn;                        // 10 matrices
   double2* lam_io = a.lam + (int64_t)b * nn;
 
   // ---- shared memory: the row lists, then matrices while they fit, else
@@ -74,8 +77,10 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
   const int64_t hn = (nn + 1) / 2;
   double* const lam = reinterpret_cast<double*>(take(hn, reinterpret_cast<double2*>(half)));
   double* const sum = reinterpret_cast<double*>(take(hn, reinterpret_cast<double2*>(half + nn)));
-  double* const VW = half + 2 * nn;
+  double* const VW = half + 2 * nn;   // a step's sums of the products
   double* const BS = half + 3 * nn;
+  double* const VWs = half + 4 * nn;  // the segment's
+  double* const BSs = half + 5 * nn;
   const auto entF = [&](int i, int c) { return heff[(int64_t)i * n + c]; };
   const auto entA = [&](int i, int c) { return hadj[(int64_t)i * n + c]; };
   const auto nonzero = [](double2 v) { return v.x != 0.0 || v.y != 0.0; };
@@ -138,8 +143,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
     put(seg, it, v);
     if (xs) put(xs, it, v);
     lam[e] = own(lam_io, it);
-    VW[e] = 0.0;
-    BS[e] = 0.0;
+    VWs[e] = 0.0;
+    BSs[e] = 0.0;
   });
   __syncthreads();
   for (int s = 0; s + 1 < a.seg_steps; ++s) {
@@ -177,15 +182,25 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
   // gradients sum: Im(conj(ab_pq) y_pq) with the items of the upper triangle,
   // Re(conj(ab_pq) y_pq) with those of the lower one (both Hermitian), the
   // bond's at every element
-  const auto products = [&](Idx e, const Item& it, const double2* ab, const double2* y) {
+  enum { kFirst, kNext, kLast };   // stage of the step
+  const auto products = [&](Idx e, const Item& it, const double2* ab, const double2* y, int stage) {
+    const auto add = [&](double* part, double* total, const auto& term) {
+      const double v = term(stage == kFirst ? 0.0 : part[e]);
+      if (stage == kLast) total[e] += v;
+      else part[e] = v;
+    };
     if (it.p != it.q) {
       const double2 av = ab[(Idx)it.p * n + it.q], yv = y[(Idx)it.p * n + it.q];
-      VW[e] = it.im ? fma(av.x, yv.x, fma(av.y, yv.y, VW[e])) : fma(av.x, yv.y, fma(-av.y, yv.x, VW[e]));
+      add(VW, VWs, [&](double v) {
+        return it.im ? fma(av.x, yv.x, fma(av.y, yv.y, v)) : fma(av.x, yv.y, fma(-av.y, yv.x, v));
+      });
     }
     const Idx k = it.im ? it.q : it.p, x = it.im ? it.p : it.q;
     if (k + 1 < n) {
       const double2 a1 = ab[k * n + x], a2 = ab[(k + 1) * n + x], v1 = y[k * n + x], v2 = y[(k + 1) * n + x];
-      BS[e] = fma(a1.x, v2.y, fma(-a1.y, v2.x, fma(a2.x, v1.y, fma(-a2.y, v1.x, BS[e]))));
+      add(BS, BSs, [&](double v) {
+        return fma(a1.x, v2.y, fma(-a1.y, v2.x, fma(a2.x, v1.y, fma(-a2.y, v1.x, v))));
+      });
     }
   };
   for (int s = a.seg_steps - 1; s >= 0; --s) {
@@ -232,27 +247,27 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
       const double yb = rhs(A, cA, madj, abA, it, u);
       sum[e] = lam[e] + yb;
       put(abB, it, fma(dt, yb, dt3 * lam[e]));
-      products(e, it, abA, y4);
+      products(e, it, abA, y4, kFirst);
     });
     __syncthreads();
     items([&](Idx e, const Item& it, int u) {
       const double yb = rhs(A, cA, madj, abB, it, u);
       sum[e] += yb;
       put(abA, it, fma(dt2, yb, dt3 * lam[e]));
-      products(e, it, abB, y3);
+      products(e, it, abB, y3, kNext);
     });
     __syncthreads();
     items([&](Idx e, const Item& it, int u) {
       const double yb = rhs(A, cA, madj, abA, it, u);
       sum[e] += yb;
       put(abB, it, fma(dt2, yb, dt6 * lam[e]));
-      products(e, it, abA, y2);
+      products(e, it, abA, y2, kNext);
     });
     __syncthreads();
     items([&](Idx e, const Item& it, int u) {
       const double yb = rhs(A, cA, madj, abB, it, u);
       lam[e] = sum[e] + yb;
-      products(e, it, abB, r);
+      products(e, it, abB, r, kLast);
     });
     __syncthreads();
   }
@@ -268,10 +283,10 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_rows_kernel(AdjArgs a,
       const int64_t up = x > k ? (int64_t)k * n + x : (int64_t)x * n + k;   // item (min, max)
       const int64_t lo = x > k ? (int64_t)x * n + k : (int64_t)k * n + x;   // item (max, min)
       if (x != k) {
-        d += x > k ? VW[up] : -VW[up];
-        g -= VW[lo];
+        d += x > k ? VWs[up] : -VWs[up];
+        g -= VWs[lo];
       }
-      w += BS[(int64_t)k * n + x];
+      w += BSs[(int64_t)k * n + x];
     }
     for (int o = 16; o > 0; o >>= 1) {
       d += __shfl_xor_sync(0xffffffffu, d, o);
