@@ -916,10 +916,11 @@ def propagate_host_pipelined(H, rho0, c_ops, e_ops, dt: float, n_steps: int, obs
     if not isinstance(e_ops, Populations) and e_ops and any(_ndim(e) != 2 for e in e_ops):
         return None
     rho_np = _host_array(rho0)
-    # a shared rho(0) in full, else the first and the last one (a whole batch
-    # that is not Hermitian, mu|g><g| say, is to be known before it runs; a
-    # pass over it takes longer than the pipeline, whose kernels look at every one)
-    if rho_np is None or not _host_hermitian(rho_np[::max(1, P - 1)] if rho_per else rho_np):
+    # one n x n comparison, of a shared rho(0) or of the first one: a batch
+    # that is not Hermitian (mu|g><g|, say) is to be known before it runs, but
+    # a pass over the batch takes longer than the pipeline, whose kernels look
+    # at every one
+    if rho_np is None or not _host_hermitian(rho_np[0] if rho_per else rho_np):
         return None
     nat.require_device()
     comp = torch.cuda.current_stream(device)
