@@ -419,7 +419,8 @@ int lime_redfield_adjoint_split(const LimeRedfieldAdjointSplitDesc* d, void* str
  *     C[z][i][j] = sum_k op(A)[z][i][k] * scale[z][k] * op(B)[z][k][j]
  * for z < batch, i < M, j < N, k < K; op conjugates when conj_a / conj_b
  * is 1.  Strides are in complex elements (row, column, batch; 0
- * broadcasts); scale is optional (NULL: 1).  Replaces the propagator and
+ * broadcasts); scale is optional (NULL: 1).  C may lie in the place of an
+ * operand of its own z while M, N <= 64.  Replaces the propagator and
  * Green's-function contractions of Redfield_solver (lime/oqs.py:169-366:
  * U(t_z) = U1 diag(exp(w t_z)) U1^-1 as one call with scale = exp(w t_z),
  * expect, correlation_2op_1t, correlation_4op_3t) and the eigenbasis

@@ -20,8 +20,9 @@
 // 4 to 5 % above that of u +- t with a rounded t = w v, the 8-fma form one 3 to
 // 4 % below; the first stage of a pass takes the former, the two others the
 // latter, and the error is at or below the one of u +- t at every length.  256
-// transforms of 4096: 722 -> 93 us, 33.5 + 4 FP64 instructions a point being
-// 78 us; 100 of length 999: 504 -> 51 us in the transforms, 3 launches for 6.
+// transforms of 4096: 719 -> 100 us, 40 + 4 FP64 instructions a point being
+// 92 us (33.5 + 4 and 91 us with 6 fma throughout); 100 of length 999: 554 -> 62
+// us, 3 launches for 6.
 
 #include "common.cuh"
 

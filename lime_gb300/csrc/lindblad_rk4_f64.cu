@@ -15,7 +15,7 @@
 // Bound: the FP64 pipe, so the work of one matrix is its DFMA count and a
 // batch smaller than the chip is spread over clusters.  Measured per RK4 step
 // against tiled GEMMs of the full Heff and L_k over one CTA: 16-site chain,
-// one instance, 58 -> 4.8 us (a stage's DFMA alone take 0.57 us of its 1.2);
+// one instance, 58 -> 5.0 us (a stage's DFMA alone take 0.57 us of its 1.2);
 // 64-site chain, 512 instances, 4.9 -> 0.24 ms; 37 levels with three dense
 // operators, 48 instances, 5.6 -> 0.61 ms.
 
@@ -578,8 +578,11 @@ static RK4Plan plan_rk4(int n, int c, int k_dense) {
 // measured, with the four barriers of dense operators 12000, against 600 for
 // a barrier of one CTA) and a launch's share.  Without dense operators the
 // entries of a row are not known here; 12 FP64 instructions an item stand for
-// a chain.  A cluster leaves every CTA at least 512 items (128 with dense
-// operators): below that the exchange costs more than it divides.
+// a chain, whatever the generator: rows with more entries (2 (n - 1)
+// instructions for real long-range couplings, 4 (n - 1) for a complex Heff,
+// listed operators) get smaller clusters than their work would pay for.  A
+// cluster leaves every CTA at least 512 items (128 with dense operators): below
+// that, on a chain, the exchange costs more than it divides.
 // Measured against one launch with one cluster size (a power of two, and one
 // CTA an instance from 77 on), 37 levels with three dense operators: 170
 // instances, 6 steps, 16.1 -> 9.9 ms; 48, 20 steps, 14.3 -> 12.3; 64-site

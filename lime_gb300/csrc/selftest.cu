@@ -1,6 +1,7 @@
 // Self-tests of the bounded device-side waits (test infrastructure; no
-// propagation).  Every wait in the propagator kernels polls an mbarrier at
-// most max_wait times; when the phase never completes the kernel ORs
+// propagation).  Every wait on an mbarrier in the propagator kernels polls it at
+// most max_wait times (the FP64 Redfield loop polls words of other SMs instead
+// and has a self-test of its own); when the phase never completes the kernel ORs
 // LIME_FLAG_TIMEOUT into its status word, releases what it holds and
 // returns, so the context stays usable.  These kernels make such waits run
 // out on purpose — on a barrier that nothing completes, or in the streaming

@@ -18,7 +18,8 @@ def _tensors():
 
 
 @pytest.mark.filterwarnings('ignore:ComplexHalf')
-@pytest.mark.parametrize('name', sorted(_tensors()))
+@pytest.mark.parametrize('name', ['conj', 'neg', 'neg_complex', 'mH', 'bfloat16', 'half', 'complex32', 'int', 'bool',
+                                  'grad', 'strided'])
 def test_tensor(name):
     x = _tensors()[name]
     got = engine._host_or_device(x, 'cuda')
