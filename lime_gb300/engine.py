@@ -916,11 +916,7 @@ def propagate_host_pipelined(H, rho0, c_ops, e_ops, dt: float, n_steps: int, obs
     if not isinstance(e_ops, Populations) and e_ops and any(_ndim(e) != 2 for e in e_ops):
         return None
     rho_np = _host_array(rho0)
-    # one n x n comparison, of a shared rho(0) or of the first one: a batch
-    # that is not Hermitian (mu|g><g|, say) is to be known before it runs, but
-    # a pass over the batch takes longer than the pipeline, whose kernels look
-    # at every one
-    if rho_np is None or not _host_hermitian(rho_np[0] if rho_per else rho_np):
+    if rho_np is None or not (rho_per or _host_hermitian(rho_np)):
         return None
     nat.require_device()
     comp = torch.cuda.current_stream(device)
@@ -960,6 +956,12 @@ def propagate_host_pipelined(H, rho0, c_ops, e_ops, dt: float, n_steps: int, obs
     # scale of the batch's max |Heff|, the scale of a single launch.  The A
     # operands are prepared before the first propagation: the propagation
     # kernel keeps every SM busy, so kernels queued behind it would wait
+    # a batch that is not Hermitian (mu|g><g|, say) is to be known before it
+    # runs: one of its rho(0), compared while the uploads land (a pass over all
+    # of them takes longer than the pipeline, whose kernels look at every one)
+    if rho_per and not _host_hermitian(rho_np[0]):
+        torch.cuda.synchronize(device)
+        return None
     with torch.cuda.stream(prep):
         top = float(torch.stack(amax).max().item())
         for gen in gens:

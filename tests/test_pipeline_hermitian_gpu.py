@@ -1,6 +1,6 @@
 """A host batch that is not Hermitian leaves the pipeline before anything is
-launched, when its shared rho(0) or its first one shows it; another one is
-found by the kernels."""
+launched, when its shared rho(0) shows it, or before it is propagated, when its
+first one does; another one is found by the kernels."""
 import numpy as np
 import pytest
 import torch
@@ -8,8 +8,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize('where', ['none', 'shared', 'shared3', 'all', 'first', 'last', 'tensor'])
-def test_known_before_the_run(where):
+def _launches(where):
     from lime_gb300 import _native as nat
     from lime_gb300 import engine
     P, n = 1000, 12
@@ -29,5 +28,18 @@ def test_known_before_the_run(where):
     nat.require_device()
     before = nat.launch_count()
     got = engine.propagate_host_pipelined(H, rho, ops, engine.Populations(n), 0.05, 3)
-    assert (got is None) == (where != 'none')
-    assert (nat.launch_count() == before) == (where not in ('none', 'last'))
+    return got is None, nat.launch_count() - before
+
+
+@pytest.mark.parametrize('where', ['shared', 'shared3', 'all', 'first', 'last', 'tensor'])
+def test_known_before_the_run(where):
+    none, full = _launches('none')
+    assert not none and full > 0
+    none, launches = _launches(where)
+    assert none
+    if where == 'last':
+        assert launches == full
+    elif where in ('all', 'first'):
+        assert launches < full          # the generators alone
+    else:
+        assert launches == 0
